@@ -13,6 +13,7 @@
 #include "lh_internal.cuh"
 
 #include "lh_kernels.cuh"
+#include "lh_fxpass.cuh"
 #include "lh_triads.cuh"
 #include "lh_xpass2.cuh"
 
@@ -136,6 +137,24 @@ static void *upload_vec(const std::vector<T> &v, cudaError_t &err) {
   return d;
 }
 
+// twiddle tables of the transforms: FP32 for the mixed form's register passes, the words of
+// lh_fx.cuh for the FP64 form's fixed-point passes
+template <typename T>
+static void *upload_twiddles(int n, cudaError_t &err) {
+  std::vector<T> t;
+  twiddles(n, t);
+  return upload_vec(t, err);
+}
+template <>
+void *upload_twiddles<double>(int n, cudaError_t &err) {
+  std::vector<int4> t(n);
+  for (int e = 0; e < n; ++e) {
+    const long double a = -2.0L * 3.14159265358979323846264338327950288L * (long double)e / (long double)n;
+    t[e] = fx_twiddle_word(cosl(a), sinl(a));
+  }
+  return upload_vec(t, err);
+}
+
 static void prof_begin(lh_handle *h, const char *name) {
   if (!h->prof) return;
   cudaEvent_t a, b;
@@ -192,19 +211,17 @@ template <typename T, int N>
 static cudaError_t set_attrs_sized(int lim) {
   cudaError_t e = cudaSuccess;
   const cudaFuncAttribute A = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  // k_xstats also holds a small static reduction array
-  if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)k_xstats<T, N>, A, lim - 1024);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)k_ib_xforce<T, N>, A, lim);
-  if constexpr (sizeof(T) == 8) {  // the Stockham passes (FP64 form and the FP64 leaf transforms)
-    if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)k_zinv_nl<T, N>, A, lim);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)k_xpass_nl<T, N>, A, lim);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)k_zfwd_nl<T, N>, A, lim);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)k_spec_zinv<T, N>, A, lim);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)k_xinv_phys<T, N>, A, lim);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)k_xfwd_phys<T, N>, A, lim);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)k_zfwd_spec<T, N>, A, lim);
+  if constexpr (sizeof(T) == 8) {  // the fixed-point passes: static arrays beside the buffers
+    const void *k[] = {(const void *)k_zinv_fx<N>, (const void *)k_xpass_fx<N>, (const void *)k_zfwd_fx<N>,
+                       (const void *)k_spec_zinv_fx<N>, (const void *)k_zfwd_spec_fx<N>, (const void *)k_xinv_phys_fx<N>,
+                       (const void *)k_xfwd_phys_fx<N>, (const void *)k_ib_xforce_fx<N>, (const void *)k_xstats_fx<N>};
+    for (const void *f : k)
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(f, A, lim - 8192);
   }
   if constexpr (sizeof(T) == 4) {  // the two-stage mixed-form passes
+    // k_xstats also holds a small static reduction array
+    if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)k_xstats<T, N>, A, lim - 1024);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)k_ib_xforce<T, N>, A, lim);
     if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)k_zinv2<N>, A, lim);
     if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)k_zfwd2<N>, A, lim);
     if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)k_spec_zinv2<N>, A, lim);
@@ -425,20 +442,14 @@ extern "C" int lh_create(const lh_config *cfg, lh_handle **out) {
   ZA(h->stage, cz * nu * nc);
   {
     if (h->prec == LH_PREC_FP64) {
-      std::vector<double> tx, tz;
-      twiddles(g.G1, tx); twiddles(g.G2, tz);
-      h->twx = upload_vec(tx, ce); if (ce == cudaSuccess) h->twz = upload_vec(tz, ce);
+      h->twx = upload_twiddles<double>(g.G1, ce); if (ce == cudaSuccess) h->twz = upload_twiddles<double>(g.G2, ce);
     } else {
-      std::vector<float> tx, tz;
-      twiddles(g.G1, tx); twiddles(g.G2, tz);
-      h->twx = upload_vec(tx, ce); if (ce == cudaSuccess) h->twz = upload_vec(tz, ce);
+      h->twx = upload_twiddles<float>(g.G1, ce); if (ce == cudaSuccess) h->twz = upload_twiddles<float>(g.G2, ce);
     }
     if (ce != cudaSuccess) { int rc = fail(h, LH_ECUDA, cudaGetErrorString(ce)); lh_destroy(h); return rc; }
   }
-  {  // FP64 twiddles for the leaves and the immersed-boundary round trip
-    std::vector<double> tx, tz;
-    twiddles(g.G1, tx); twiddles(g.G2, tz);
-    h->twx64 = upload_vec(tx, ce); if (ce == cudaSuccess) h->twz64 = upload_vec(tz, ce);
+  {  // the leaves' tables
+    h->twx64 = upload_twiddles<double>(g.G1, ce); if (ce == cudaSuccess) h->twz64 = upload_twiddles<double>(g.G2, ce);
     if (ce != cudaSuccess) { int rc = fail(h, LH_ECUDA, cudaGetErrorString(ce)); lh_destroy(h); return rc; }
   }
   // immersed boundaries
@@ -567,13 +578,11 @@ extern "C" int lh_create(const lh_config *cfg, lh_handle **out) {
     h->twv[1][0] = h->twv[1][1] = nullptr;
     if (mb && ce == cudaSuccess) {
       if (h->prec == LH_PREC_FP64) {
-        std::vector<double> tx, tz;
-        twiddles(cfg->Ngal1c, tx); twiddles(cfg->Ngal2c, tz);
-        h->twv[1][0] = upload_vec(tx, ce); if (ce == cudaSuccess) h->twv[1][1] = upload_vec(tz, ce);
+        h->twv[1][0] = upload_twiddles<double>(cfg->Ngal1c, ce);
+        if (ce == cudaSuccess) h->twv[1][1] = upload_twiddles<double>(cfg->Ngal2c, ce);
       } else {
-        std::vector<float> tx, tz;
-        twiddles(cfg->Ngal1c, tx); twiddles(cfg->Ngal2c, tz);
-        h->twv[1][0] = upload_vec(tx, ce); if (ce == cudaSuccess) h->twv[1][1] = upload_vec(tz, ce);
+        h->twv[1][0] = upload_twiddles<float>(cfg->Ngal1c, ce);
+        if (ce == cudaSuccess) h->twv[1][1] = upload_twiddles<float>(cfg->Ngal2c, ce);
       }
     }
     if (ce != cudaSuccess) { int rc = fail(h, LH_ECUDA, cudaGetErrorString(ce)); lh_destroy(h); return rc; }
@@ -1048,11 +1057,11 @@ static int launch_zinv(lh_handle *h, const Geo &g, int nslots, const void *twz) 
     dim3 grid((g.N1h + P::KB - 1) / P::KB, nslots, 3);
     KL("k_zinv_nl", k_zinv2<N><<<grid, P::NT, P::SMEM, h->st>>>(h->u1, h->u2, h->u3, (float2 *)h->A, g,
                                                                 (const float2 *)twz));
-  } else {  // FP64: Stockham
-    constexpr int KB = kb_zinv<V>(N);
+  } else {  // FP64: fixed point
+    constexpr int KB = fx_kbz(N);
     dim3 grid((g.N1h + KB - 1) / KB, nslots, 3);
-    KL("k_zinv_nl", k_zinv_nl<T, N><<<grid, LH_ZINV_THREADS, 2 * (size_t)KB * N * sizeof(V), h->st>>>(
-                        h->u1, h->u2, h->u3, (V *)h->A, g, (const V *)twz));
+    KL("k_zinv_nl", k_zinv_fx<N><<<grid, fx_zt(N), fx_smem(N, KB), h->st>>>(h->u1, h->u2, h->u3, (double2 *)h->A, g,
+                                                                           (const int4 *)twz));
   }
   return LH_OK;
 }
@@ -1069,12 +1078,12 @@ static int launch_xpass(lh_handle *h, const Geo &g, int nslots, int doCFL, const
     dim3 grid(g.G2 / 2, nslots);
     KL("k_xpass_nl", k_xpass3<N><<<grid, P::NT, P::SMEM, h->st>>>((const float2 *)h->A, (float2 *)h->B, g,
                                                                   (const float2 *)twx, doCFL, h->sc, capslot, (float *)h->cap));
-  } else {  // FP64: Stockham
+  } else {  // FP64: fixed point
     static_assert(sizeof(T) == 8, "the mixed x pass has a register form for every compiled length");
-    constexpr int PB = pb_xpass<V>(N);
+    constexpr int PB = fx_pbx(N);
     dim3 grid((g.G2 / 2 + PB - 1) / PB, nslots);
-    KL("k_xpass_nl", k_xpass_nl<T, N><<<grid, LH_XPASS_THREADS, 8 * (size_t)PB * N * sizeof(V), h->st>>>(
-                         (const V *)h->A, (V *)h->B, g, (const V *)twx, doCFL, h->sc, capslot, (T *)h->cap));
+    KL("k_xpass_nl", k_xpass_fx<N><<<grid, fx_xt(N), fx_smem(N, 4 * PB), h->st>>>(
+                         (const double2 *)h->A, (double2 *)h->B, g, (const int4 *)twx, doCFL, h->sc, capslot, (double *)h->cap));
   }
   return LH_OK;
 }
@@ -1087,12 +1096,12 @@ static int launch_zfwd(lh_handle *h, const Geo &g, int nslots, const void *twz) 
     KL("k_zfwd_nl", k_zfwd2<N><<<grid, P::NTH, P::SMEM, h->st>>>(
                         (const float2 *)h->B, g, (const float2 *)twz, (float2 *)h->N1xz, (float2 *)h->N2xz,
                         (float2 *)h->N3xz, (float2 *)h->uvf, (float2 *)h->vvc, (float2 *)h->wvf));
-  } else {  // FP64: Stockham
-    constexpr int KB = kb_zfwd<V>(N);
+  } else {  // FP64: fixed point
+    constexpr int KB = fx_kbf(N);
     dim3 grid((g.N1h + KB - 1) / KB, nslots);
-    KL("k_zfwd_nl", k_zfwd_nl<T, N><<<grid, LH_ZFWD_THREADS, 8 * (size_t)KB * N * sizeof(V), h->st>>>(
-                        (const V *)h->B, g, (const V *)twz, (V *)h->N1xz, (V *)h->N2xz, (V *)h->N3xz, (V *)h->uvf,
-                        (V *)h->vvc, (V *)h->wvf));
+    KL("k_zfwd_nl", k_zfwd_fx<N><<<grid, fx_zt(N), fx_smem(N, 4 * KB), h->st>>>(
+                        (const double2 *)h->B, g, (const int4 *)twz, (double2 *)h->N1xz, (double2 *)h->N2xz,
+                        (double2 *)h->N3xz, (double2 *)h->uvf, (double2 *)h->vvc, (double2 *)h->wvf));
   }
   return LH_OK;
 }
@@ -1153,27 +1162,25 @@ static int launch_spec_zinv(lh_handle *h, const void *spec, void *Ascr, int npl,
     using P = zp2<N>;
     dim3 g1((h->g.N1h + P::KB - 1) / P::KB, npl);
     KL("k_spec_zinv", k_spec_zinv2<N><<<g1, P::NT, P::SMEM, h->st>>>((const float2 *)spec, (float2 *)Ascr, h->g, (const float2 *)twz));
-  } else {  // FP64: Stockham
-    constexpr int KB = kb_zinv<V>(N);
+  } else {  // FP64: fixed point
+    constexpr int KB = fx_kbz(N);
     dim3 g1((h->g.N1h + KB - 1) / KB, npl);
-    KL("k_spec_zinv", k_spec_zinv<T, N><<<g1, NTHR_H, 2 * (size_t)KB * N * sizeof(V), h->st>>>((const double2 *)spec, (V *)Ascr, h->g, (const V *)twz));
+    KL("k_spec_zinv", k_spec_zinv_fx<N><<<g1, fx_zt(N), fx_smem(N, KB), h->st>>>((const double2 *)spec, (double2 *)Ascr, h->g, (const int4 *)twz));
   }
   return LH_OK;
 }
-template <typename T, int N>
+template <int N>
 static int launch_xinv_phys(lh_handle *h, const void *Ascr, double *phys, int npl, const void *twx) {
-  typedef typename C2<T>::t V;
-  constexpr int PB = 4 * pb_xpass<V>(N);
+  constexpr int PB = fx_pbl(N);
   dim3 g2((h->g.G2 / 2 + PB - 1) / PB, npl);
-  KL("k_xinv_phys", k_xinv_phys<T, N><<<g2, NTHR_H, 2 * (size_t)PB * N * sizeof(V), h->st>>>((const V *)Ascr, phys, h->g, (const V *)twx));
+  KL("k_xinv_phys", k_xinv_phys_fx<N><<<g2, fx_xt(N), fx_smem(N, PB), h->st>>>((const double2 *)Ascr, phys, h->g, (const int4 *)twx));
   return LH_OK;
 }
-template <typename T, int N>
+template <int N>
 static int launch_xfwd_phys(lh_handle *h, const double *phys, void *Bscr, int npl, const void *twx) {
-  typedef typename C2<T>::t V;
-  constexpr int PB = 4 * pb_xpass<V>(N);
+  constexpr int PB = fx_pbl(N);
   dim3 g1((h->g.G2 / 2 + PB - 1) / PB, npl);
-  KL("k_xfwd_phys", k_xfwd_phys<T, N><<<g1, NTHR_H, 2 * (size_t)PB * N * sizeof(V), h->st>>>(phys, (V *)Bscr, h->g, (const V *)twx));
+  KL("k_xfwd_phys", k_xfwd_phys_fx<N><<<g1, fx_xt(N), fx_smem(N, PB), h->st>>>(phys, (double2 *)Bscr, h->g, (const int4 *)twx));
   return LH_OK;
 }
 template <typename T, int N>
@@ -1183,41 +1190,45 @@ static int launch_zfwd_spec(lh_handle *h, const void *Bscr, void *spec, int npl,
     using P = zp2<N>;
     dim3 g2((h->g.N1h + P::KB - 1) / P::KB, npl);
     KL("k_zfwd_spec", k_zfwd_spec2<N><<<g2, P::NT, P::SMEM, h->st>>>((const float2 *)Bscr, (float2 *)spec, h->g, (const float2 *)twz));
-  } else {  // FP64: Stockham
-    constexpr int KB = kb_zinv<V>(N);
+  } else {  // FP64: fixed point
+    constexpr int KB = fx_kbz(N);
     dim3 g2((h->g.N1h + KB - 1) / KB, npl);
-    KL("k_zfwd_spec", k_zfwd_spec<T, N><<<g2, NTHR_H, 2 * (size_t)KB * N * sizeof(V), h->st>>>((const V *)Bscr, (double2 *)spec, h->g, (const V *)twz));
+    KL("k_zfwd_spec", k_zfwd_spec_fx<N><<<g2, fx_zt(N), fx_smem(N, KB), h->st>>>((const double2 *)Bscr, (double2 *)spec, h->g, (const int4 *)twz));
   }
   return LH_OK;
 }
 
 template <typename T, int N>
 static int launch_ib_xforce(lh_handle *h, int npl) {
-  typedef typename C2<T>::t V;
-  constexpr int PB = 4 * pb_xpass<V>(N);
-  dim3 g2((h->g.G2 / 2 + PB - 1) / PB, npl);
-  KL("k_ib_xforce", k_ib_xforce<T, N><<<g2, NTHR_H, 2 * (size_t)PB * N * sizeof(V), h->st>>>(
-                        (const V *)h->A, (V *)h->B, h->g, (const V *)h->twx, h->d_ibrec, h->d_iboff, (const T *)h->cap, h->sc));
+  if constexpr (sizeof(T) == 4) {
+    constexpr int PB = 4 * pb_xpass<float2>(N);
+    dim3 g2((h->g.G2 / 2 + PB - 1) / PB, npl);
+    KL("k_ib_xforce", k_ib_xforce<float, N><<<g2, NTHR_H, 2 * (size_t)PB * N * sizeof(float2), h->st>>>(
+                          (const float2 *)h->A, (float2 *)h->B, h->g, (const float2 *)h->twx, h->d_ibrec, h->d_iboff, (const float *)h->cap, h->sc));
+  } else {  // FP64: fixed point
+    constexpr int PB = fx_pbl(N);
+    dim3 g2((h->g.G2 / 2 + PB - 1) / PB, npl);
+    KL("k_ib_xforce", k_ib_xforce_fx<N><<<g2, fx_xt(N), fx_smem(N, PB), h->st>>>(
+                          (const double2 *)h->A, (double2 *)h->B, h->g, (const int4 *)h->twx, h->d_ibrec, h->d_iboff, (const double *)h->cap, h->sc));
+  }
   return LH_OK;
 }
-template <typename T>
 static int spec_to_phys(lh_handle *h, const double2 *spec, double *phys, int npl, void *Ascr, const void *twx,
                         const void *twz) {
   int rc = LH_EINVAL;
-  LH_DISPATCH(h->g.G2, rc = launch_spec_zinv<T, N>(h, spec, Ascr, npl, twz));
+  LH_DISPATCH(h->g.G2, rc = (launch_spec_zinv<double, N>(h, spec, Ascr, npl, twz)));
   if (rc) return rc;
   rc = LH_EINVAL;
-  LH_DISPATCH(h->g.G1, rc = launch_xinv_phys<T, N>(h, Ascr, phys, npl, twx));
+  LH_DISPATCH(h->g.G1, rc = launch_xinv_phys<N>(h, Ascr, phys, npl, twx));
   return rc;
 }
-template <typename T>
 static int phys_to_spec(lh_handle *h, const double *phys, double2 *spec, int npl, void *Bscr, const void *twx,
                         const void *twz) {
   int rc = LH_EINVAL;
-  LH_DISPATCH(h->g.G1, rc = launch_xfwd_phys<T, N>(h, phys, Bscr, npl, twx));
+  LH_DISPATCH(h->g.G1, rc = launch_xfwd_phys<N>(h, phys, Bscr, npl, twx));
   if (rc) return rc;
   rc = LH_EINVAL;
-  LH_DISPATCH(h->g.G2, rc = launch_zfwd_spec<T, N>(h, Bscr, spec, npl, twz));
+  LH_DISPATCH(h->g.G2, rc = (launch_zfwd_spec<double, N>(h, Bscr, spec, npl, twz)));
   return rc;
 }
 
@@ -1449,12 +1460,19 @@ extern "C" int lh_profile_steps(lh_handle *h, int nsteps, lh_kernel_time *out, i
 // the sums of stats.f90 (k_xstats), per plane class
 template <typename T, int N>
 static int launch_xstats(lh_handle *h, const Geo &g, int nslots, const void *twx) {
-  typedef typename C2<T>::t V;
-  constexpr int PB = pb_xpass<V>(N);
-  dim3 grid((g.G2 / 2 + PB - 1) / PB, nslots);
-  KL("k_xstats", k_xstats<T, N><<<grid, NTHR_H, 8 * (size_t)PB * N * sizeof(V), h->st>>>(
-                     (const V *)h->A, g, (const V *)twx, h->st_pl, h->st_cd, h->st_ncl, h->st_dnx, h->st_dnz,
-                     h->st_ntx));
+  if constexpr (sizeof(T) == 4) {
+    constexpr int PB = pb_xpass<float2>(N);
+    dim3 grid((g.G2 / 2 + PB - 1) / PB, nslots);
+    KL("k_xstats", k_xstats<T, N><<<grid, NTHR_H, 8 * (size_t)PB * N * sizeof(float2), h->st>>>(
+                       (const float2 *)h->A, g, (const float2 *)twx, h->st_pl, h->st_cd, h->st_ncl, h->st_dnx, h->st_dnz,
+                       h->st_ntx));
+  } else {  // FP64: fixed point
+    constexpr int PB = fx_pbx(N);
+    dim3 grid((g.G2 / 2 + PB - 1) / PB, nslots);
+    KL("k_xstats", k_xstats_fx<N><<<grid, fx_xt(N), fx_smem(N, 3 * PB), h->st>>>(
+                       (const double2 *)h->A, g, (const int4 *)twx, h->st_pl, h->st_cd, h->st_ncl, h->st_dnx, h->st_dnz,
+                       h->st_ntx));
+  }
   return LH_OK;
 }
 template <typename T>
@@ -1568,7 +1586,7 @@ static int pressure_wx_stats(lh_handle *h, int nhc, int n2c) {
     const int nb = std::min(h->cond_chunk, h->n_cond - b0);
     KL("k_cond_spec", k_cond_spec<<<dim3((g.ncolF + LH_STAT_THREADS - 1) / LH_STAT_THREADS, nb), LH_STAT_THREADS, 0,
                                      h->st>>>(h->u2, h->u3, h->p, g, h->d_cond_list + b0, spec));
-    if ((rc = spec_to_phys<double>(h, spec, phys, nb, h->A, fp64_tw(h, true), fp64_tw(h, false)))) return rc;
+    if ((rc = spec_to_phys(h, spec, phys, nb, h->A, fp64_tw(h, true), fp64_tw(h, false)))) return rc;
     KL("k_cond_phys", k_cond_phys<<<dim3((cells + LH_STAT_THREADS - 1) / LH_STAT_THREADS, nb), LH_STAT_THREADS, 0,
                                      h->st>>>(phys, h->d_cond_list + b0, g.G1, g.G2, h->st_dnx, h->st_dnz,
                                               h->st_ncl + 1, h->st_cd4));
@@ -1714,14 +1732,14 @@ extern "C" int lh_four_to_phys(lh_handle *h, const void *spec, void *phys, int n
   if (!h || !spec || !phys || nplanes <= 0) return LH_EINVAL;
   const size_t need = sizeof(double2) * (size_t)nplanes * h->g.G2 * h->g.N1h;
   if (need > h->Abytes) return fail(h, LH_EINVAL, "too many planes for the scratch buffer");
-  return spec_to_phys<double>(h, (const double2 *)spec, (double *)phys, nplanes, h->A, fp64_tw(h, true), fp64_tw(h, false));
+  return spec_to_phys(h, (const double2 *)spec, (double *)phys, nplanes, h->A, fp64_tw(h, true), fp64_tw(h, false));
 }
 
 extern "C" int lh_phys_to_four(lh_handle *h, const void *phys, void *spec, int nplanes) {
   if (!h || !spec || !phys || nplanes <= 0) return LH_EINVAL;
   const size_t need = sizeof(double2) * (size_t)nplanes * h->g.G2 * h->g.N1h;
   if (need > h->Bbytes) return fail(h, LH_EINVAL, "too many planes for the scratch buffer");
-  return phys_to_spec<double>(h, (const double *)phys, (double2 *)spec, nplanes, h->B, fp64_tw(h, true), fp64_tw(h, false));
+  return phys_to_spec(h, (const double *)phys, (double2 *)spec, nplanes, h->B, fp64_tw(h, true), fp64_tw(h, false));
 }
 
 // ---------------------------------------------------------------------------

@@ -1,13 +1,13 @@
-// lh_kernels.cuh — CUDA kernels of the RK3 substep (FP64 plain form; transforms
-// templated on the transform precision).
+// lh_kernels.cuh — CUDA kernels of the RK3 substep outside its transform passes, which are in
+// lh_fxpass.cuh (FP64 form, fixed point) and lh_xpass2.cuh (mixed form, FP32).
 //
 // Per substep (littleharsh.f90:174-217):
-//   k_zinv_nl   : stagger interpolation (FOU3D.f90:427-474) fused into the inverse z
+//   k_zinv_fx, k_zinv2  : stagger interpolation (FOU3D.f90:427-474) fused into the inverse z
 //                 transforms of the six velocity planes of every level (cft, iopt>=0)
-//   k_xpass_nl  : inverse x transforms (rft, iopt>=0), physical products
+//   k_xpass_fx, k_xpass2 / k_xpass3 : inverse x transforms (rft, iopt>=0), physical products
 //                 (ops_in_planes2, FOU3D.f90:2090-2251), CFL maxima (dtc_calc), forward x
 //                 transforms (rft, iopt<0) of the products
-//   k_zfwd_nl   : forward z transforms (cft, iopt<0) + der_x/der_z (FOU3D.f90:476-593):
+//   k_zfwd_fx, k_zfwd2  : forward z transforms (cft, iopt<0) + der_x/der_z (FOU3D.f90:476-593):
 //                 N_xz of u, v, w and the y-flux products uv, vv, wv
 //   k_dt        : dt = min(2.5 dtv, CFL dtc) on the device (FOU3D.f90:291-297)
 //   k_helm_uw   : RHS0_u1/u3 + der_yu_h + du += -gRK N + solveU_W, one thread per column
@@ -15,8 +15,8 @@
 //   k_meanflow  : flowrate_corr on mode (0,0) (constant flow rate)
 //   k_press2    : divergence + solveP (LUsolP with the stored factors, k_build_dg) + v_corr
 //                 + divergence of the corrected field in the third substep (max |div| -> err)
-//   k_ib_du(_mx), k_spec_zinv, k_ib_xforce, k_zfwd_spec : immersed-boundary forcing of du
-//                 (imm_bounds_u/v, FOU3D.f90:806-998) when the geometry has posts
+//   k_ib_du(_mx), k_spec_zinv(_fx, 2), k_ib_xforce(_fx), k_zfwd_spec(_fx, 2) : immersed-boundary
+//                 forcing of du (imm_bounds_u/v, FOU3D.f90:806-998) when the geometry has posts
 //   Mixed form (LH_PREC_MIXED): FP32 transforms, and k_helm_u_mx2 / k_helm_v_mx2 solve
 //   the Helmholtz systems for the increment in FP32 on top of the FP64 state.
 // On request: k_xstats, k_wx_stats, k_spectra, k_slip (statistics), k_band_io, k_transpose
@@ -77,9 +77,6 @@ __device__ __forceinline__ T warp_max(T v) {
 #ifndef LH_BUDGET_XPASS
 #define LH_BUDGET_XPASS 24576
 #endif
-#ifndef LH_BUDGET_ZFWD
-#define LH_BUDGET_ZFWD 49152
-#endif
 __host__ __device__ constexpr int lh_clamp(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 template <typename V> __host__ __device__ constexpr int kb_zinv(int n) {
   return lh_clamp(LH_BUDGET_ZINV / (2 * n * (int)sizeof(V)), 1, 16);
@@ -87,16 +84,14 @@ template <typename V> __host__ __device__ constexpr int kb_zinv(int n) {
 template <typename V> __host__ __device__ constexpr int pb_xpass(int n) {
   return lh_clamp(LH_BUDGET_XPASS / (8 * n * (int)sizeof(V)), 1, 8);
 }
-template <typename V> __host__ __device__ constexpr int kb_zfwd(int n) {
-  return lh_clamp(LH_BUDGET_ZFWD / (8 * n * (int)sizeof(V)), 1, 8);
-}
 
-// ============================================================================
-// T1: inverse z transforms of the velocity planes (with stagger interpolation).
-// grid: x = kx group of KB lines, y = level slot (u-levels then v-levels), z = field.
-// A layout: [(slot*3 + f)][l][kx], l = 0..G2-1, kx = 0..N1h-1.
-// Lines are interleaved in shared memory (element l of line kk at l*KB + kk).
-// ============================================================================
+// Transform intermediates. A (after the inverse z pass): [(slot*3 + f)][l][kx], l = 0..G2-1,
+// kx = 0..N1h-1. B (after the x pass): [pslot][l/2][kx][l%2] (the two rows of a pair interleaved,
+// so that the z pass reads a few columns of a row pair as one contiguous run); pslot = slot*4 + p
+// (u levels), nuI*4 + (slot-nuI)*2 + p (v). The x pass carries each pair of rows (l, l+1) of a
+// field in one complex line (row l in .x, row l+1 in .y after the transform). Optional capture:
+// physical velocities of selected levels, [cap][f][l][m].
+
 // Levels loaded ahead in the y sweeps of the column solves (0: a plain loop). Without it
 // a sweep's loads wait for the previous level's stores (the compiler cannot separate the
 // addresses), one memory latency per level. Deeper prefetch costs registers, i.e. resident
@@ -119,218 +114,6 @@ template <typename V> __host__ __device__ constexpr int kb_zfwd(int n) {
 #ifndef LH_PRESS_MINB
 #define LH_PRESS_MINB 1
 #endif
-#ifndef LH_ZINV_THREADS
-#define LH_ZINV_THREADS 256
-#endif
-#ifndef LH_ZFWD_THREADS
-#define LH_ZFWD_THREADS 256
-#endif
-template <typename T, int N>
-__global__ void __launch_bounds__(LH_ZINV_THREADS) k_zinv_nl(const double2 *__restrict__ u1, const double2 *__restrict__ u2,
-                                                  const double2 *__restrict__ u3, typename C2<T>::t *__restrict__ A,
-                                                  Geo g, const typename C2<T>::t *__restrict__ twz) {
-  typedef typename C2<T>::t V;
-  constexpr int KB = kb_zinv<V>(N);
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  V *b0 = reinterpret_cast<V *>(smem_raw);
-  V *b1 = b0 + KB * N;
-  const int slot = zinv_slot(g, blockIdx.y), f = blockIdx.z, kx0 = blockIdx.x * KB;
-  const bool isU = slot < g.nuI;
-  const int q = slot_level(g, slot, isU);
-  const int nc = g.ncolF;
-  for (int i = threadIdx.x; i < KB * N; i += blockDim.x) b0[i] = czero<V>();
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < g.N2 * KB; idx += blockDim.x) {
-    const int r = idx / KB, kk = idx - r * KB, kx = kx0 + kk;
-    if (kx >= g.N1h) continue;
-    const int c = gcol(g, r, kx);
-    V v;
-    if (isU) {
-      if (f == 0) { const double2 x = u1[(size_t)q * nc + c]; v.x = to_t<T>(x.x); v.y = to_t<T>(x.y); }
-      else if (f == 2) { const double2 x = u3[(size_t)q * nc + c]; v.x = to_t<T>(x.x); v.y = to_t<T>(x.y); }
-      else {  // interp_v: v faces -> centre q
-        const double2 v0 = u2[(size_t)q * nc + c], vm = u2[(size_t)(q - 1) * nc + c];
-        if (sizeof(T) == 8) {
-          const double a = g.iua[q], b = g.iub[q];
-          v.x = (T)(a * v0.x + b * vm.x);
-          v.y = (T)(a * v0.y + b * vm.y);
-        } else {
-          const T a = (T)g.iuaf[q], b = (T)g.iubf[q];
-          v.x = a * to_t<T>(v0.x) + b * to_t<T>(vm.x);
-          v.y = a * to_t<T>(v0.y) + b * to_t<T>(vm.y);
-        }
-      }
-    } else {
-      if (f == 1) { const double2 x = u2[(size_t)q * nc + c]; v.x = to_t<T>(x.x); v.y = to_t<T>(x.y); }
-      else {  // interp_u: centres -> face q
-        const double2 *src = (f == 0) ? u1 : u3;
-        const double2 up = src[(size_t)(q + 1) * nc + c], u0 = src[(size_t)q * nc + c];
-        if (sizeof(T) == 8) {
-          const double a = g.iva[q], b = g.ivb[q];
-          v.x = (T)(a * up.x + b * u0.x);
-          v.y = (T)(a * up.y + b * u0.y);
-        } else {
-          const T a = (T)g.ivaf[q], b = (T)g.ivbf[q];
-          v.x = a * to_t<T>(up.x) + b * to_t<T>(u0.x);
-          v.y = a * to_t<T>(up.y) + b * to_t<T>(u0.y);
-        }
-      }
-    }
-    b0[prow(g, r) * KB + kk] = v;
-  }
-  __syncthreads();
-  V *res = line_fft<true, N, KB, true>(b0, b1, twz);
-  V *dst = A + (size_t)(slot * 3 + f) * N * g.N1h;
-  for (int idx = threadIdx.x; idx < N * KB; idx += blockDim.x) {
-    const int l = idx / KB, kk = idx - l * KB, kx = kx0 + kk;
-    if (kx < g.N1h) dst[(size_t)l * g.N1h + kx] = res[l * KB + kk];
-  }
-}
-
-// ============================================================================
-// T2: x pass. PB row pairs per block; each pair of rows (l, l+1) of a field is
-// carried by one complex line (row l in .x, row l+1 in .y after the transform).
-// B layout: [pslot][l/2][kx][l%2] (the two rows of a pair interleaved, so that the z pass
-// reads a few columns of a row pair as one contiguous run); pslot = slot*4 + p (u levels),
-// nuI*4 + (slot-nuI)*2 + p (v).
-// capture (optional): physical velocities of selected levels, [cap][f][l][m].
-// ============================================================================
-// x pass: one row pair per block (FP32) in 4 warps: a Stockham pass over the few lines
-// of a block then spreads evenly over the threads (the fastest of a sweep at C1)
-#ifndef LH_XPASS_THREADS
-#define LH_XPASS_THREADS 128
-#endif
-template <typename T, int N>
-__global__ void __launch_bounds__(LH_XPASS_THREADS) k_xpass_nl(const typename C2<T>::t *__restrict__ A,
-                                                   typename C2<T>::t *__restrict__ B, Geo g,
-                                                   const typename C2<T>::t *__restrict__ twx, int doCFL,
-                                                   DevScalars *sc, const int *__restrict__ capslot,
-                                                   T *__restrict__ cap) {
-  typedef typename C2<T>::t V;
-  constexpr int PB = pb_xpass<V>(N);
-  constexpr int G1 = N, H = N / 2;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int G2 = g.G2, N1h = g.N1h;
-  V *b0 = reinterpret_cast<V *>(smem_raw);
-  V *b1 = b0 + 4 * PB * G1;
-  const int slot = blockIdx.y;
-  const bool isU = slot < g.nuI;
-  const int q = slot_level(g, slot, isU);
-  const int l0 = blockIdx.x * PB * 2;
-  const int npairs = min(PB, (G2 - l0) / 2);
-  const size_t fstride = (size_t)G2 * N1h;
-  const V *Af = A + (size_t)slot * 3 * fstride;
-  // gather Hermitian-completed lines of the 3 fields: line f*PB + pb. One work item per
-  // retained x-mode k writes element k (a + i b) and element G1 - k (conj(a) + i conj(b));
-  // elements N1h .. G1 - N1h (the dealiasing band) are zero. N1 = 2 (Ngal1 / 3) (lh_create
-  // checks it), so N1h = G1 / 3 + 1 is a compile-time constant here.
-  constexpr int NK = G1 / 3 + 1, NZ = G1 - 2 * NK + 1;
-  static_assert(NK <= H, "retained x-modes below the Nyquist index");
-  for (int idx = threadIdx.x; idx < 3 * PB * NK; idx += blockDim.x) {
-    const int line = idx / NK, k = idx - line * NK;
-    const int f = line / PB, pb = line - f * PB;
-    V zd = czero<V>(), zc = czero<V>();
-    if (pb < npairs) {
-      const int l = l0 + 2 * pb;
-      V a = Af[f * fstride + (size_t)l * NK + k];
-      V b = Af[f * fstride + (size_t)(l + 1) * NK + k];
-      if (k == 0) { a.y = 0; b.y = 0; }
-      zd.x = a.x - b.y; zd.y = a.y + b.x;   // a + i b
-      zc.x = a.x + b.y; zc.y = -a.y + b.x;  // conj(a) + i conj(b)
-    }
-    b0[line * G1 + k] = zd;
-    if (k > 0) b0[line * G1 + G1 - k] = zc;
-  }
-  for (int idx = threadIdx.x; idx < 3 * PB * NZ; idx += blockDim.x) {
-    const int line = idx / NZ, m = idx - line * NZ;
-    b0[line * G1 + NK + m] = czero<V>();
-  }
-  __syncthreads();
-  V *res = line_fft<true, N, 3 * PB, false>(b0, b1, twx);
-  V *oth = (res == b0) ? b1 : b0;
-  if (capslot) {
-    const int cs = capslot[slot];
-    if (cs >= 0) {
-      for (int idx = threadIdx.x; idx < 3 * PB * G1; idx += blockDim.x) {
-        const int line = idx / G1, m = idx - line * G1;
-        const int f = line / PB, pb = line - f * PB;
-        if (pb >= npairs) continue;
-        const int l = l0 + 2 * pb;
-        T *cp = cap + ((size_t)cs * 3 + f) * (size_t)G2 * G1;
-        const V z = res[idx];
-        cp[(size_t)l * G1 + m] = z.x;
-        cp[(size_t)(l + 1) * G1 + m] = z.y;
-      }
-    }
-  }
-  T m1 = 0, m2 = 0, m3 = 0;
-  const T thv = isU ? (T)0 : (sizeof(T) == 8 ? (T)g.thv[q] : (T)g.thvf[q]);
-  for (int idx = threadIdx.x; idx < PB * G1; idx += blockDim.x) {
-    const int pb = idx / G1, m = idx - pb * G1;
-    const V u = res[(0 * PB + pb) * G1 + m], v = res[(1 * PB + pb) * G1 + m], w = res[(2 * PB + pb) * G1 + m];
-    const bool valid = pb < npairs;
-    if (isU) {
-      V p0, p1, p2, p3;
-      p0.x = u.x * u.x; p0.y = u.y * u.y;
-      p1.x = u.x * w.x; p1.y = u.y * w.y;
-      p2.x = v.x * v.x; p2.y = v.y * v.y;
-      p3.x = w.x * w.x; p3.y = w.y * w.y;
-      oth[(0 * PB + pb) * G1 + m] = p0;
-      oth[(1 * PB + pb) * G1 + m] = p1;
-      oth[(2 * PB + pb) * G1 + m] = p2;
-      oth[(3 * PB + pb) * G1 + m] = p3;
-      if (valid && doCFL) {
-        m1 = nmax(m1, nmax(fabs(u.x), fabs(u.y)));
-        m3 = nmax(m3, nmax(fabs(w.x), fabs(w.y)));
-      }
-    } else {
-      V p0, p1;
-      p0.x = u.x * v.x; p0.y = u.y * v.y;
-      p1.x = w.x * v.x; p1.y = w.y * v.y;
-      oth[(0 * PB + pb) * G1 + m] = p0;
-      oth[(1 * PB + pb) * G1 + m] = p1;
-      if (valid && doCFL) m2 = nmax(m2, nmax(fabs(v.x), fabs(v.y)) * thv);
-    }
-  }
-  if (doCFL) {
-    m1 = warp_max(m1); m2 = warp_max(m2); m3 = warp_max(m3);
-    if ((threadIdx.x & 31) == 0) {
-      if (isU) { atomic_max_pos(&sc->u1m, to_d(m1)); atomic_max_pos(&sc->u3m, to_d(m3)); }
-      else atomic_max_pos(&sc->u2m, to_d(m2));
-    }
-  }
-  __syncthreads();
-  V *pres = isU ? line_fft<false, N, 4 * PB, false>(oth, res, twx) : line_fft<false, N, 2 * PB, false>(oth, res, twx);
-  const int nprod = isU ? 4 : 2;
-  const T s1 = (T)1 / (T)G1;
-  const int pbase = isU ? slot * 4 : g.nuI * 4 + (slot - g.nuI) * 2;
-  // separate the two rows of each pair, keep kx = 0..N1h-1; kx fastest (coalesced rows).
-  // N1 = 2 (Ngal1 / 3) (lh_create checks it), so N1h = G1 / 3 + 1 is a compile-time
-  // constant here and the index split needs no runtime division.
-  // One work item per x-mode k writes both rows of the pair, which sit next to each other
-  // in B (one 16-byte store in the mixed form).
-  constexpr int NH = G1 / 3 + 1;
-  for (int idx = threadIdx.x; idx < nprod * PB * NH; idx += blockDim.x) {
-    const int k = idx % NH;
-    const int r2 = idx / NH;
-    const int pb = r2 % PB, p = r2 / PB;
-    if (pb >= npairs) continue;
-    const V *L = pres + (p * PB + pb) * G1;
-    const V z = L[k], zc = cconj(L[k == 0 ? 0 : G1 - k]);
-    V o0, o1;
-    o0.x = (T)0.5 * (z.x + zc.x) * s1; o0.y = (T)0.5 * (z.y + zc.y) * s1;
-    o1.x = (T)0.5 * (z.y - zc.y) * s1; o1.y = (T)-0.5 * (z.x - zc.x) * s1;  // -0.5 i (z - zc)
-    if (k == 0) { o0.y = 0; o1.y = 0; }
-    V *dst = B + (((size_t)(pbase + p) * (G2 / 2) + (l0 >> 1) + pb) * N1h + k) * 2;
-    if constexpr (sizeof(T) == 4) {
-      *reinterpret_cast<float4 *>(dst) = make_float4(o0.x, o0.y, o1.x, o1.y);
-    } else {
-      dst[0] = o0;
-      dst[1] = o1;
-    }
-  }
-}
-
 // ============================================================================
 // Statistics (stats.f90:1-250) of one plane class: the x pass's gather and inverse
 // transform, then the plane sums (per level) and the tile-conditioned sums (wall-band
@@ -340,46 +123,12 @@ __global__ void __launch_bounds__(LH_XPASS_THREADS) k_xpass_nl(const typename C2
 // conditioned sums add the ntilex tiles of a row in registers first.
 // pl: [11][nu] (quantities 0-8 here); cd: [9][ncl][dnz][dnx].
 // ============================================================================
-template <typename T, int N>
-__global__ void __launch_bounds__(NTHR) k_xstats(const typename C2<T>::t *__restrict__ A, Geo g,
-                                                 const typename C2<T>::t *__restrict__ twx, double *__restrict__ pl,
-                                                 double *__restrict__ cd, int ncl, int dnx, int dnz, int ntx) {
-  typedef typename C2<T>::t V;
-  constexpr int PB = pb_xpass<V>(N);
-  constexpr int G1 = N, H = N / 2;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ double red[NTHR / 32][6];
-  const int G2 = g.G2, N1h = g.N1h;
-  V *b0 = reinterpret_cast<V *>(smem_raw);
-  V *b1 = b0 + 4 * PB * G1;
-  const int slot = blockIdx.y;
-  const bool isU = slot < g.nuI;
-  const int q = slot_level(g, slot, isU);
-  const int l0 = blockIdx.x * PB * 2;
-  const int npairs = min(PB, (G2 - l0) / 2);
-  const size_t fstride = (size_t)G2 * N1h;
-  const V *Af = A + (size_t)slot * 3 * fstride;
-  for (int idx = threadIdx.x; idx < 3 * PB * G1; idx += blockDim.x) {
-    const int line = idx / G1, m = idx - line * G1;
-    const int f = line / PB, pb = line - f * PB;
-    V z = czero<V>();
-    if (pb < npairs) {
-      const int l = l0 + 2 * pb;
-      int k = m;
-      bool conjpart = false;
-      if (m > H) { k = G1 - m; conjpart = true; }
-      if (k < N1h) {
-        V a = Af[f * fstride + (size_t)l * N1h + k];
-        V b = Af[f * fstride + (size_t)(l + 1) * N1h + k];
-        if (k == 0 || k == H) { a.y = 0; b.y = 0; }
-        if (!conjpart) { z.x = a.x - b.y; z.y = a.y + b.x; }
-        else { z.x = a.x + b.y; z.y = -a.y + b.x; }
-      }
-    }
-    b0[idx] = z;
-  }
-  __syncthreads();
-  const V *res = line_fft<true, N, 3 * PB, false>(b0, b1, twx);
+template <int N, int PB, typename V>
+__device__ __forceinline__ void xstats_sums(const V *__restrict__ res, const Geo &g, double *__restrict__ pl,
+                                            double *__restrict__ cd, int ncl, int dnx, int dnz, int ntx, bool isU, int q,
+                                            int l0, int npairs) {
+  constexpr int G1 = N;
+  __shared__ double red[16][6];
   // plane sums
   double s[6] = {0, 0, 0, 0, 0, 0};
   for (int idx = threadIdx.x; idx < PB * G1; idx += blockDim.x) {
@@ -430,83 +179,46 @@ __global__ void __launch_bounds__(NTHR) k_xstats(const typename C2<T>::t *__rest
   }
 }
 
-// ============================================================================
-// T3: forward z transforms + der_x/der_z. grid: x = kx group (KB), y = level slot.
-// u level: products uu, uw, vv, ww -> N1xz, N3xz, vvc.   v level: uv, wv -> N2xz, uvf, wvf.
-// Outputs are complex in the transform precision (TO = T).
-// ============================================================================
-template <typename T, int N, int NP>
-__device__ __forceinline__ void zfwd_body(const typename C2<T>::t *__restrict__ B, const Geo &g,
-                                          const typename C2<T>::t *__restrict__ twz, int slot, int q, int pbase,
-                                          typename C2<T>::t *o0, typename C2<T>::t *o1, typename C2<T>::t *o2,
-                                          typename C2<T>::t *o3, typename C2<T>::t *o4, typename C2<T>::t *o5) {
-  typedef typename C2<T>::t V;
-  constexpr int KB = kb_zfwd<V>(N);
-  constexpr int NL = NP * KB;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int N1h = g.N1h, N2 = g.N2;
-  const int kx0 = blockIdx.x * KB;
-  V *b0 = reinterpret_cast<V *>(smem_raw);
-  V *b1 = b0 + 4 * KB * N;
-  // line = p*KB + kk; element l at l*NL + line. B holds the rows of a pair next to each
-  // other ([product][l/2][kx][l%2]): the KB columns of a row pair are 2*KB contiguous values.
-  for (int idx = threadIdx.x; idx < N * NL; idx += blockDim.x) {
-    const int h = idx & 1;
-    int rest = idx >> 1;
-    const int kk = rest % KB;
-    rest /= KB;
-    const int lp = rest % (N / 2), p = rest / (N / 2);
-    const int l = 2 * lp + h, kx = kx0 + kk;
-    V z = czero<V>();
-    if (kx < N1h) z = B[(((size_t)(pbase + p) * (N / 2) + lp) * N1h + kx) * 2 + h];
-    b0[l * NL + p * KB + kk] = z;
-  }
-  __syncthreads();
-  V *res = line_fft<false, N, NL, true>(b0, b1, twz);
-  const T s2 = (T)1 / (T)N;
-  const size_t off = (size_t)q * g.ncolF;
-  for (int idx = threadIdx.x; idx < N2 * KB; idx += blockDim.x) {
-    const int r = idx / KB, kk = idx - r * KB, kx = kx0 + kk;
-    if (kx >= N1h) continue;
-    const int row = prow(g, r);
-    const int c = gcol(g, r, kx), rg = grow(g, r);
-    const T kxv = sizeof(T) == 8 ? (T)g.k1x[kx] : (T)g.k1xf[kx];
-    const T kzv = sizeof(T) == 8 ? (T)g.k1z[rg] : (T)g.k1zf[rg];
-    const bool zr = (r == N2 / 2);  // der_x/der_z zero the kz = -N2/2 row
-    if (NP == 4) {
-      const V uu = cscale(res[row * NL + 0 * KB + kk], s2), uw = cscale(res[row * NL + 1 * KB + kk], s2);
-      const V vv = cscale(res[row * NL + 2 * KB + kk], s2), ww = cscale(res[row * NL + 3 * KB + kk], s2);
-      V n1 = czero<V>(), n3 = czero<V>();
-      if (!zr) {
-        n1 = cadd(cimul(kxv, uu), cimul(kzv, uw));
-        n3 = cadd(cimul(kxv, uw), cimul(kzv, ww));
-      }
-      o0[off + c] = n1;  // N1xz
-      o2[off + c] = n3;  // N3xz
-      o4[off + c] = vv;  // vvc
-    } else {
-      const V uv = cscale(res[row * NL + 0 * KB + kk], s2), wv = cscale(res[row * NL + 1 * KB + kk], s2);
-      V n2 = czero<V>();
-      if (!zr) n2 = cadd(cimul(kxv, uv), cimul(kzv, wv));
-      o1[off + c] = n2;  // N2xz
-      o3[off + c] = uv;  // uvf
-      o5[off + c] = wv;  // wvf
-    }
-  }
-}
-
 template <typename T, int N>
-__global__ void __launch_bounds__(LH_ZFWD_THREADS) k_zfwd_nl(const typename C2<T>::t *__restrict__ B, Geo g,
-                                                  const typename C2<T>::t *__restrict__ twz,
-                                                  typename C2<T>::t *__restrict__ N1xz, typename C2<T>::t *__restrict__ N2xz,
-                                                  typename C2<T>::t *__restrict__ N3xz, typename C2<T>::t *__restrict__ uvf,
-                                                  typename C2<T>::t *__restrict__ vvc, typename C2<T>::t *__restrict__ wvf) {
+__global__ void __launch_bounds__(NTHR) k_xstats(const typename C2<T>::t *__restrict__ A, Geo g,
+                                                 const typename C2<T>::t *__restrict__ twx, double *__restrict__ pl,
+                                                 double *__restrict__ cd, int ncl, int dnx, int dnz, int ntx) {
+  typedef typename C2<T>::t V;
+  constexpr int PB = pb_xpass<V>(N);
+  constexpr int G1 = N, H = N / 2;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int G2 = g.G2, N1h = g.N1h;
+  V *b0 = reinterpret_cast<V *>(smem_raw);
+  V *b1 = b0 + 4 * PB * G1;
   const int slot = blockIdx.y;
   const bool isU = slot < g.nuI;
   const int q = slot_level(g, slot, isU);
-  const int pbase = isU ? slot * 4 : g.nuI * 4 + (slot - g.nuI) * 2;
-  if (isU) zfwd_body<T, N, 4>(B, g, twz, slot, q, pbase, N1xz, N2xz, N3xz, uvf, vvc, wvf);
-  else zfwd_body<T, N, 2>(B, g, twz, slot, q, pbase, N1xz, N2xz, N3xz, uvf, vvc, wvf);
+  const int l0 = blockIdx.x * PB * 2;
+  const int npairs = min(PB, (G2 - l0) / 2);
+  const size_t fstride = (size_t)G2 * N1h;
+  const V *Af = A + (size_t)slot * 3 * fstride;
+  for (int idx = threadIdx.x; idx < 3 * PB * G1; idx += blockDim.x) {
+    const int line = idx / G1, m = idx - line * G1;
+    const int f = line / PB, pb = line - f * PB;
+    V z = czero<V>();
+    if (pb < npairs) {
+      const int l = l0 + 2 * pb;
+      int k = m;
+      bool conjpart = false;
+      if (m > H) { k = G1 - m; conjpart = true; }
+      if (k < N1h) {
+        V a = Af[f * fstride + (size_t)l * N1h + k];
+        V b = Af[f * fstride + (size_t)(l + 1) * N1h + k];
+        if (k == 0 || k == H) { a.y = 0; b.y = 0; }
+        if (!conjpart) { z.x = a.x - b.y; z.y = a.y + b.x; }
+        else { z.x = a.x + b.y; z.y = -a.y + b.x; }
+      }
+    }
+    b0[idx] = z;
+  }
+  __syncthreads();
+  const V *res = line_fft<true, N, 3 * PB, false>(b0, b1, twx);
+  xstats_sums<N, PB>(res, g, pl, cd, ncl, dnx, dnz, ntx, isU, q, l0, npairs);
 }
 
 // ============================================================================
@@ -2246,9 +1958,9 @@ __global__ void k_transpose(const double2 *__restrict__ src, double2 *__restrict
 }
 
 // ============================================================================
-// Generic plane transforms (leaves lh_four_to_phys / lh_phys_to_four and the
-// immersed-boundary round trip of du). spec [plane][N2][N1h] complex128, phys
-// [plane][G2][G1] double, scratch A/B [plane][l][kx] in the transform precision.
+// Plane transforms of lh_four_to_phys_noalloc (FP64 Stockham: its scratch holds FP64 tables
+// that every call makes on the device). spec [plane][N2][N1h] complex128, phys [plane][G2][G1]
+// double, scratch A [plane][l][kx]. The handles' leaves run in lh_fxpass.cuh.
 // ============================================================================
 template <typename T, int N>
 __global__ void __launch_bounds__(NTHR) k_spec_zinv(const double2 *__restrict__ spec, typename C2<T>::t *__restrict__ A,
@@ -2315,75 +2027,6 @@ __global__ void __launch_bounds__(NTHR) k_xinv_phys(const typename C2<T>::t *__r
     const int l = l0 + 2 * pb;
     P[(size_t)l * G1 + m] = to_d(res[idx].x);
     P[(size_t)(l + 1) * G1 + m] = to_d(res[idx].y);
-  }
-}
-
-template <typename T, int N>
-__global__ void __launch_bounds__(NTHR) k_xfwd_phys(const double *__restrict__ phys, typename C2<T>::t *__restrict__ B,
-                                                    Geo g, const typename C2<T>::t *__restrict__ twx) {
-  typedef typename C2<T>::t V;
-  constexpr int PB = 4 * pb_xpass<V>(N);
-  constexpr int G1 = N;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int G2 = g.G2, N1h = g.N1h;
-  V *b0 = reinterpret_cast<V *>(smem_raw);
-  V *b1 = b0 + PB * G1;
-  const int pl = blockIdx.y, l0 = blockIdx.x * PB * 2;
-  const int npairs = min(PB, (G2 - l0) / 2);
-  const double *P = phys + (size_t)pl * G2 * G1;
-  for (int idx = threadIdx.x; idx < PB * G1; idx += blockDim.x) {
-    const int pb = idx / G1, m = idx - pb * G1;
-    V z = czero<V>();
-    if (pb < npairs) {
-      const int l = l0 + 2 * pb;
-      z.x = to_t<T>(P[(size_t)l * G1 + m]);
-      z.y = to_t<T>(P[(size_t)(l + 1) * G1 + m]);
-    }
-    b0[idx] = z;
-  }
-  __syncthreads();
-  V *res = line_fft<false, N, PB, false>(b0, b1, twx);
-  const T s1 = (T)1 / (T)G1;
-  for (int idx = threadIdx.x; idx < PB * 2 * N1h; idx += blockDim.x) {
-    const int k = idx % N1h, rest = idx / N1h;
-    const int half = rest & 1, pb = rest >> 1;
-    if (pb >= npairs) continue;
-    const V *L = res + pb * G1;
-    const V z = L[k], zc = cconj(L[(G1 - k) % G1]);
-    V o;
-    if (!half) { o.x = (T)0.5 * (z.x + zc.x) * s1; o.y = (T)0.5 * (z.y + zc.y) * s1; }
-    else { o.x = (T)0.5 * (z.y - zc.y) * s1; o.y = (T)-0.5 * (z.x - zc.x) * s1; }
-    if (k == 0) o.y = 0;
-    B[((size_t)pl * G2 + l0 + 2 * pb + half) * N1h + k] = o;
-  }
-}
-
-template <typename T, int N>
-__global__ void __launch_bounds__(NTHR) k_zfwd_spec(const typename C2<T>::t *__restrict__ B, double2 *__restrict__ spec,
-                                                    Geo g, const typename C2<T>::t *__restrict__ twz) {
-  typedef typename C2<T>::t V;
-  constexpr int KB = kb_zinv<V>(N);
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int N1h = g.N1h, N2 = g.N2;
-  V *b0 = reinterpret_cast<V *>(smem_raw);
-  V *b1 = b0 + KB * N;
-  const int pl = blockIdx.y, kx0 = blockIdx.x * KB;
-  for (int idx = threadIdx.x; idx < N * KB; idx += blockDim.x) {
-    const int l = idx / KB, kk = idx - l * KB, kx = kx0 + kk;
-    V z = czero<V>();
-    if (kx < N1h) z = B[((size_t)pl * N + l) * N1h + kx];
-    b0[idx] = z;
-  }
-  __syncthreads();
-  V *res = line_fft<false, N, KB, true>(b0, b1, twz);
-  const double s2 = 1.0 / (double)N;
-  double2 *S = spec + (size_t)pl * g.ncol;
-  for (int idx = threadIdx.x; idx < N2 * KB; idx += blockDim.x) {
-    const int r = idx / KB, kk = idx - r * KB, kx = kx0 + kk;
-    if (kx >= N1h) continue;
-    const V t = res[prow(g, r) * KB + kk];
-    double2 o; o.x = to_d(t.x) * s2; o.y = to_d(t.y) * s2;
-    S[r * N1h + kx] = o;
   }
 }
 
