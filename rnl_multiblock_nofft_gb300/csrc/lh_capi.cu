@@ -423,7 +423,8 @@ extern "C" int lh_create(const lh_config *cfg, lh_handle **out) {
   ZA(h->N2xz, vs * nv * nc); ZA(h->uvf, vs * nv * nc); ZA(h->wvf, vs * nv * nc);
   // a3s: the FP64 solves' upper factors; in the mixed form the previous nonlinear term of mode
   // (0,0) in FP64 (k_helm00_pcr: 6 x nu doubles; nc >= 8 always)
-  ZA(h->psi, cz * g.np * nc); ZA(h->a3s, sizeof(double) * nu * nc); ZA(h->a3v, sizeof(double) * nv * nc);
+  const size_t split = h->prec == LH_PREC_FP64 && g.nvc < LH_H64_SPLIT ? 2 : 1;  // k_helm64<., 1, 1>: factors per field and part
+  ZA(h->psi, cz * g.np * nc); ZA(h->a3s, split * split * sizeof(double) * nu * nc); ZA(h->a3v, split * sizeof(double) * nv * nc);
   ZA(h->mfw, sizeof(double) * 6 * (size_t)(g.nn + 3));
   h->Abytes = h->Bbytes = 0;
   for (int vi = 0; vi < h->nviews; ++vi) {
@@ -619,6 +620,10 @@ extern "C" int lh_create(const lh_config *cfg, lh_handle **out) {
     if (smem_optin(&lim) || cudaFuncSetAttribute((const void *)k_press3<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
         cudaFuncSetAttribute((const void *)k_press3<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
         cudaFuncSetAttribute((const void *)k_press3<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
+        cudaFuncSetAttribute((const void *)k_helm64<false, 2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
+        cudaFuncSetAttribute((const void *)k_helm64<false, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
+        cudaFuncSetAttribute((const void *)k_helm64<true, 1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
+        cudaFuncSetAttribute((const void *)k_helm64<true, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
         cudaFuncSetAttribute((const void *)k_helm_u_mx3<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
         cudaFuncSetAttribute((const void *)k_helm_u_mx3<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
         cudaFuncSetAttribute((const void *)k_helm_u_mx3<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
@@ -1260,6 +1265,30 @@ static size_t press_smem(const Geo &g, int pf, int tb) {
   return sizeof(double) * (((size_t)g.nu + g.nv + 1) & ~(size_t)1) + sizeof(double) * 6 * (size_t)(pf + 1) * tb;
 }
 
+// the FP64 form's Helmholtz solves: one lane per column while the columns fill the SMs, one per
+// column, field and part below (k_helm64)
+static bool helm64_split(const lh_handle *h) { return h->g.nvc < LH_H64_SPLIT; }
+static void launch_helm64_v(lh_handle *h, int kRK, cudaStream_t st) {
+  Helm64Args a = {{(double *)h->u2, nullptr}, {(double *)h->Nu2, nullptr}, {(const double *)h->N2xz, nullptr},
+                  {(const double *)h->vvc, nullptr}, (const double *)h->p, h->a3v, h->ib ? h->d_ibslot_v : nullptr,
+                  (const double *)h->duib, kRK};
+  const int nl = h->g.nv, n = h->g.nvc;
+  if (helm64_split(h)) k_helm64<true, 1, 1><<<(2 * n + LH_H64_T - 1) / LH_H64_T, LH_H64_T, helm64_smem(true, 1, 1, nl), st>>>(a, h->g, h->sc);
+  else k_helm64<true, 1, 2><<<(n + LH_H64_T - 1) / LH_H64_T, LH_H64_T, helm64_smem(true, 1, 2, nl), st>>>(a, h->g, h->sc);
+}
+static void launch_helm64_uw(lh_handle *h, int kRK) {
+  Helm64Args a = {{(double *)h->u1, (double *)h->u3}, {(double *)h->Nu1, (double *)h->Nu3},
+                  {(const double *)h->N1xz, (const double *)h->N3xz}, {(const double *)h->uvf, (const double *)h->wvf},
+                  (const double *)h->p, h->a3s, h->ib ? h->d_ibslot_u : nullptr, (const double *)h->duib, kRK};
+  const int nl = h->g.nu, n = h->g.nvc;
+  if (helm64_split(h)) {
+    const dim3 grid((2 * n + LH_H64_T - 1) / LH_H64_T, 2);
+    k_helm64<false, 1, 1><<<grid, LH_H64_T, helm64_smem(false, 1, 1, nl), h->st>>>(a, h->g, h->sc);
+  } else {
+    k_helm64<false, 2, 2><<<(n + LH_H64_T - 1) / LH_H64_T, LH_H64_T, helm64_smem(false, 2, 2, nl), h->st>>>(a, h->g, h->sc);
+  }
+}
+
 template <typename T>
 static int substep_launches_t(lh_handle *h, int kRK) {
   typedef typename C2<T>::t V;
@@ -1268,7 +1297,6 @@ static int substep_launches_t(lh_handle *h, int kRK) {
   if (rc) return rc;
   if (kRK == 1) KL("k_dt", k_dt<<<1, 32, 0, h->st>>>(g, h->sc));
   const int nb = (g.ncol + NTHR_H - 1) / NTHR_H;
-  const int nbu = (g.nvc + h->tb_uw - 1) / h->tb_uw, nbv = (g.nvc + h->tb_v - 1) / h->tb_v;
   if (h->ib) {
     dim3 gd(nb, h->nib);
     if (h->prec == LH_PREC_FP64) {
@@ -1307,8 +1335,7 @@ static int substep_launches_t(lh_handle *h, int kRK) {
   }
   if (!fork) prof_begin(h, "k_helm_v");
   if (h->prec == LH_PREC_FP64) {
-    k_helm_v<T><<<nbv, h->tb_v, 0, sv>>>(h->u2, (double2 *)h->Nu2, (const V *)h->N2xz, (const V *)h->vvc, h->p,
-                                         h->a3v, g, h->sc, kRK, h->ib ? h->d_ibslot_v : nullptr, (const double2 *)h->duib);
+    launch_helm64_v(h, kRK, sv);
   } else {
     const int nb2v = (2 * g.nvc + h->tb_v - 1) / h->tb_v;
     const size_t sm = staged_smem(g.nv, h->pf_v, h->tb_v);
@@ -1337,10 +1364,7 @@ static int substep_launches_t(lh_handle *h, int kRK) {
   }
   if (fork) CK(cudaEventRecord(h->ev_join, h->st2));
   if (h->prec == LH_PREC_FP64) {
-    KL("k_helm_uw", k_helm_uw<T><<<nbu, h->tb_uw, 0, h->st>>>(h->u1, h->u3, (double2 *)h->Nu1, (double2 *)h->Nu3,
-                                                           (const V *)h->N1xz, (const V *)h->N3xz, (const V *)h->uvf,
-                                                           (const V *)h->wvf, h->p, h->a3s, g, h->sc, kRK,
-                                                           h->ib ? h->d_ibslot_u : nullptr, (const double2 *)h->duib));
+    KL("k_helm_uw", launch_helm64_uw(h, kRK));
   } else {
     const int nb2u = (2 * g.nvc + h->tb_uw - 1) / h->tb_uw;
     const size_t sm = staged_smem(g.nu, h->pf_uw, h->tb_uw);

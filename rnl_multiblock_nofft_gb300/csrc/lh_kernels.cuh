@@ -249,203 +249,261 @@ __global__ void k_reset_cfl(DevScalars *sc) {
   if (threadIdx.x == 0 && blockIdx.x == 0) { sc->u1m = 0ull; sc->u2m = 0ull; sc->u3m = 0ull; }
 }
 
-// ============================================================================
-// Helmholtz u and w (shared matrix), one thread per column.
-// Levels q = 0 .. nu-1 (ghosts at 0 and nu-1). For interior q the right-hand side
-// is u + dt * du with du = RHS0 (laplacian, -cRK Nu_old, -dRK grad p, -dRK mpgx on
-// (0,0)) - gRK Nu_new, Nu_new = N_xz + d/dy(uv or wv); Nu_new replaces Nu.
-// The forward sweep stores y in u and the upper factor in `a3s`; the backward
-// sweep writes the solution in place. At immersed-boundary levels du is read from
-// `duib` (assembled and forced beforehand) instead of being formed here.
-// ============================================================================
 template <typename VN>
 __device__ __forceinline__ double2 ld2(const VN &v) { return make_double2((double)v.x, (double)v.y); }
 
-template <typename TN>
-__global__ void __launch_bounds__(NTHR) k_helm_uw(double2 *__restrict__ u1, double2 *__restrict__ u3,
-                                                  double2 *__restrict__ Nu1, double2 *__restrict__ Nu3,
-                                                  const typename C2<TN>::t *__restrict__ N1xz, const typename C2<TN>::t *__restrict__ N3xz,
-                                                  const typename C2<TN>::t *__restrict__ uvf, const typename C2<TN>::t *__restrict__ wvf,
-                                                  const double2 *__restrict__ p, double *__restrict__ a3s, Geo g,
-                                                  const DevScalars *__restrict__ sc, int kRK,
-                                                  const int *__restrict__ ibslot_u, const double2 *__restrict__ duib) {
-  const int vc = blockIdx.x * blockDim.x + threadIdx.x;
-  const int nc = g.ncol;
-  if (vc >= g.nvc) return;
-  int c, bd;
-  vcol_of(g, vc, c, bd);
-  const int qlo = g.bq[bd][0], qhi = g.bq[bd][1];
-  const int r = c / g.N1h, kx = c - r * g.N1h;
-  const double k2x = g.k2x[kx], k2z = g.k2z[r];
-  const double C1 = g.aRK[kRK - 1] / g.Re, C2 = -g.cRK[kRK - 1], dR = g.dRK[kRK - 1];
-  const double G = -g.gRK[kRK - 1];
-  const double dt = sc->dt;
-  const double beta = g.bRK[kRK - 1] * dt / g.Re;
-  const double C3x = -dR * g.k1x[kx], C3z = -dR * g.k1z[r];  // imaginary parts of -dRK*k1F
-  const double mp = (c == 0) ? -dR * sc->mpgx : 0.0;
-  const int nu = g.nu;
-  const double *d0 = g.d2u, *d1 = g.d2u + nu, *d2 = g.d2u + 2 * nu;
-  // first row: [1, gw(b,1)], rhs 0
-  double a3raw = g.gw[bd][0];
-  double a2p = 1.0;  // 1/a2(0)
-  double2 y1 = czero<double2>(), y3 = czero<double2>();
-  const size_t o0 = (size_t)qlo * nc + c;
-  double2 um1 = u1[o0], u0 = u1[o0 + nc];
-  double2 wm1 = u3[o0], w0 = u3[o0 + nc];
-  u1[o0] = y1;
-  u3[o0] = y3;
-  double2 uvm = ld2(uvf[o0]), wvm = ld2(wvf[o0]);
-  for (int q = qlo + 1; q <= qhi - 1; ++q) {
-    const size_t o = (size_t)q * nc + c;
-    const double2 up1 = u1[o + nc], wp1 = u3[o + nc];
-    const double2 uvq = ld2(uvf[o]), wvq = ld2(wvf[o]);
-    double2 du1, du3;
-    const int ibs = ibslot_u ? ibslot_u[q] : -1;
-    if (ibs < 0) {
-      const double a = d0[q], dg = (k2x + k2z) + d1[q], cc = d2[q];
-      double2 L1, L3;
-      L1.x = (a * um1.x + dg * u0.x) + cc * up1.x; L1.y = (a * um1.y + dg * u0.y) + cc * up1.y;
-      L3.x = (a * wm1.x + dg * w0.x) + cc * wp1.x; L3.y = (a * wm1.y + dg * w0.y) + cc * wp1.y;
-      const double2 pj = p[(size_t)(q - 1) * nc + c];
-      const double2 no1 = Nu1[o], no3 = Nu3[o];
-      du1.x = (C1 * L1.x + C2 * no1.x) + (-C3x * pj.y);
-      du1.y = (C1 * L1.y + C2 * no1.y) + (C3x * pj.x);
-      du3.x = (C1 * L3.x + C2 * no3.x) + (-C3z * pj.y);
-      du3.y = (C1 * L3.y + C2 * no3.y) + (C3z * pj.x);
-      du1.x += mp;
-      const double th = g.thu[q];
-      const double2 x1 = ld2(N1xz[o]), x3 = ld2(N3xz[o]);
-      double2 n1, n3;
-      n1.x = x1.x + (uvq.x - uvm.x) * th * g.dd; n1.y = x1.y + (uvq.y - uvm.y) * th * g.dd;
-      n3.x = x3.x + (wvq.x - wvm.x) * th * g.dd; n3.y = x3.y + (wvq.y - wvm.y) * th * g.dd;
-      Nu1[o] = n1;
-      Nu3[o] = n3;
-      du1.x = du1.x + G * n1.x; du1.y = du1.y + G * n1.y;
-      du3.x = du3.x + G * n3.x; du3.y = du3.y + G * n3.y;
-    } else {
-      du1 = duib[((size_t)ibs * 3 + 0) * nc + c];
-      du3 = duib[((size_t)ibs * 3 + 2) * nc + c];
-    }
-    double2 rhs1, rhs3;
-    rhs1.x = u0.x + dt * du1.x; rhs1.y = u0.y + dt * du1.y;
-    rhs3.x = w0.x + dt * du3.x; rhs3.y = w0.y + dt * du3.y;
-    const double a1 = -beta * d0[q];
-    const double a2 = 1.0 - beta * ((d1[q] + k2x) + k2z);
-    const double a3p = a3raw * a2p;  // a3'(q-1)
-    a3s[(size_t)(q - 1) * nc + c] = a3p;
-    a2p = 1.0 / (a2 - a1 * a3p);
-    y1.x = (rhs1.x - a1 * y1.x) * a2p; y1.y = (rhs1.y - a1 * y1.y) * a2p;
-    y3.x = (rhs3.x - a1 * y3.x) * a2p; y3.y = (rhs3.y - a1 * y3.y) * a2p;
-    u1[o] = y1;
-    u3[o] = y3;
-    a3raw = -beta * d2[q];
-    um1 = u0; u0 = up1; wm1 = w0; w0 = wp1;
-    uvm = uvq; wvm = wvq;
-  }
-  {  // last row: [gw(b,2), 1], rhs 0
-    const int q = qhi;
-    const double a1 = g.gw[bd][1];
-    const double a3p = a3raw * a2p;
-    a3s[(size_t)(q - 1) * nc + c] = a3p;
-    a2p = 1.0 / (1.0 - a1 * a3p);
-    y1.x = (0.0 - a1 * y1.x) * a2p; y1.y = (0.0 - a1 * y1.y) * a2p;
-    y3.x = (0.0 - a1 * y3.x) * a2p; y3.y = (0.0 - a1 * y3.y) * a2p;
-    u1[(size_t)q * nc + c] = y1;
-    u3[(size_t)q * nc + c] = y3;
-  }
-  double2 x1 = y1, x3 = y3;
-  for (int q = qhi - 1; q >= qlo; --q) {
-    const size_t o = (size_t)q * nc + c;
-    const double a3p = a3s[o];
-    const double2 yy1 = u1[o], yy3 = u3[o];
-    x1.x = yy1.x - a3p * x1.x; x1.y = yy1.y - a3p * x1.y;
-    x3.x = yy3.x - a3p * x3.x; x3.y = yy3.y - a3p * x3.y;
-    u1[o] = x1;
-    u3[o] = x3;
-  }
+// cp.async copies from global to shared memory (16, 8 and 4 bytes), their commit groups and waits
+__device__ __forceinline__ void cpa16(void *dst, const void *src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
 }
+__device__ __forceinline__ void cpa8(void *dst, const void *src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cpa4(void *dst, const void *src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cpa_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cpa_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 // ============================================================================
-// Helmholtz v, one thread per column. Levels q = 0 .. nv-1 (walls at both ends).
+// Helmholtz solves of the FP64 form (RHS0 + N assembly + LU + both sweeps of one column
+// segment). For interior q the right-hand side is u + dt * du with du = RHS0 (laplacian,
+// -cRK Nu_old, -dRK grad p, -dRK mpgx on (0,0)) - gRK Nu_new, Nu_new = N_xz + d/dy(flux);
+// Nu_new replaces Nu. The forward sweep stores y in the field and the upper factor in a3s; the
+// backward sweep writes the solution in place. At immersed-boundary levels du is read from
+// `duib` (assembled and forced beforehand) instead of being formed here.
+//
+// A lane carries NF fields (u and w share their matrix) and NP parts (real, imaginary) of one
+// column; field blockIdx.y + 0 .. NF-1, part (lane % (2 / NP)).
+//  - Large channels, <2, 2> and v <1, 2>: bound by the FP64 pipe (2 operations a clock and SM), so
+//    one lane does everything that shares the factorisation, and the operations are few: the
+//    row l of -dt / Re L serves the matrix (I + bRK l) and the right-hand side (-aRK l u), and
+//    dt is folded into the other coefficients. u/w 93 -> 66 and v 65 -> 42 operations a column level.
+//  - Small channels, <1, 1>: bound by the serial chain of a level (reciprocal and two fused
+//    operations, ~1/3 of a microsecond) and by the FP64 issue of the few SMs that hold the
+//    columns, so the components spread over four times as many lanes (each repeats the
+//    factorisation).
+// The level's inputs come D levels ahead through a cp.async ring in shared memory. 32-thread
+// blocks spread the columns evenly over the 152 SMs (1032 blocks at 256 x 256: 6.8 a SM).
+// Measured at 256 x 256 x 301 with posts / 32 x 32 x 153, ms per step, against one lane per
+// column with all operations in the reference's order: u/w 5.63 -> 4.32 / 1.32 -> 0.49, v 3.94 -> 2.89 / 0.89 -> 0.49
+// (both run together in the step: FP64 pipe 82-86 % busy).
 // ============================================================================
-template <typename TN>
-__global__ void __launch_bounds__(NTHR) k_helm_v(double2 *__restrict__ u2, double2 *__restrict__ Nu2,
-                                                 const typename C2<TN>::t *__restrict__ N2xz, const typename C2<TN>::t *__restrict__ vvc,
-                                                 const double2 *__restrict__ p, double *__restrict__ a3s, Geo g,
-                                                 const DevScalars *__restrict__ sc, int kRK,
-                                                 const int *__restrict__ ibslot_v, const double2 *__restrict__ duib) {
-  const int vc = blockIdx.x * blockDim.x + threadIdx.x;
+#define LH_H64_D 2   // levels ahead
+#define LH_H64_T 32  // threads per block
+// columns below which the components spread over lanes: twice the lanes that one warp per SM holds
+#define LH_H64_SPLIT 2432
+template <int NP> struct Part;
+template <> struct Part<2> { typedef double2 t; };
+template <> struct Part<1> { typedef double t; };
+__device__ __forceinline__ double &comp(double2 &v, int s) { return s ? v.y : v.x; }
+__device__ __forceinline__ double &comp(double &v, int) { return v; }
+__device__ __forceinline__ void cpa_part(double2 *d, const double *s) { cpa16(d, s); }
+__device__ __forceinline__ void cpa_part(double *d, const double *s) { cpa8(d, s); }
+
+struct Helm64Args {
+  double *u[2];          // the fields (v: [0])
+  double *Nu[2];         // previous nonlinear terms
+  const double *X[2];    // N_xz
+  const double *F[2];    // y-flux
+  const double *p;
+  double *a3s;           // upper factors [field group][level][column]
+  const int *ibslot;
+  const double *duib;
+  int kRK;
+};
+__host__ __device__ constexpr int helm64_entries(bool V, int NF) { return V ? 5 : 1 + 4 * NF; }
+// bytes: the level tables (row of -dt / Re L without k^2, d/dy factor, immersed slot) and the ring
+__host__ __device__ constexpr size_t helm64_smem(bool V, int NF, int NP, int nlev) {
+  return (((size_t)nlev * 36 + 15) & ~(size_t)15) +
+         (size_t)helm64_entries(V, NF) * (LH_H64_D + 1) * LH_H64_T * 8 * NP;
+}
+
+// V: the wall-normal velocity (levels at the faces; gradient and flux differences across them)
+template <bool V, int NF, int NP>
+__global__ void __launch_bounds__(LH_H64_T) k_helm64(Helm64Args a, Geo g, const DevScalars *__restrict__ sc) {
+  typedef typename Part<NP>::t T;
+  constexpr int D = LH_H64_D, NS = D + 1, NT = LH_H64_T, NE = helm64_entries(V, NF);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int nlev = V ? g.nv : g.nu, kRK = a.kRK;
+  double *t1 = reinterpret_cast<double *>(smem_raw), *t2 = t1 + nlev, *t3 = t2 + nlev, *tth = t3 + nlev;
+  int *tib = reinterpret_cast<int *>(tth + nlev);
+  T *ring = reinterpret_cast<T *>(smem_raw + (((size_t)nlev * 36 + 15) & ~(size_t)15));
+  const double dt = sc->dt;
+  const double unit = -dt / g.Re;  // the tables hold -dt / Re L
+  {
+    const double *d2 = V ? g.d2v : g.d2u, *th = V ? g.thv : g.thu;
+    for (int i = threadIdx.x; i < nlev; i += NT) {
+      t1[i] = unit * d2[i]; t2[i] = unit * d2[nlev + i]; t3[i] = unit * d2[2 * nlev + i];
+      tth[i] = th[i] * g.dd;
+      tib[i] = a.ibslot ? a.ibslot[i] : -1;
+    }
+  }
+  __syncthreads();
+  const int lane = blockIdx.x * NT + threadIdx.x;
+  const int vc = NP == 2 ? lane : lane >> 1, part = NP == 2 ? 0 : lane & 1;
   const int nc = g.ncol;
   if (vc >= g.nvc) return;
   int c, bd;
   vcol_of(g, vc, c, bd);
-  const int qlo = g.bq[bd][2], qhi = g.bq[bd][3];
+  const int qlo = g.bq[bd][V ? 2 : 0], qhi = g.bq[bd][V ? 3 : 1];
   const int r = c / g.N1h, kx = c - r * g.N1h;
-  const double k2x = g.k2x[kx], k2z = g.k2z[r];
-  const double C1 = g.aRK[kRK - 1] / g.Re, C2 = -g.cRK[kRK - 1], dR = g.dRK[kRK - 1];
-  const double G = -g.gRK[kRK - 1];
-  const double dt = sc->dt;
-  const double beta = g.bRK[kRK - 1] * dt / g.Re;
-  const int nv = g.nv;
-  const double *d0 = g.d2v, *d1 = g.d2v + nv, *d2 = g.d2v + 2 * nv;
-  double a3raw = 0.0, a2p = 1.0;
-  double2 y = czero<double2>();
-  const size_t o0 = (size_t)qlo * nc + c;
-  double2 vm1 = u2[o0], v0 = u2[o0 + nc];
-  u2[o0] = y;
-  double2 vvq = ld2(vvc[o0 + nc]);  // vv at u level q (interior starts at qlo + 1)
-  for (int q = qlo + 1; q <= qhi - 1; ++q) {
-    const size_t o = (size_t)q * nc + c;
-    const double2 vp1 = u2[o + nc];
-    const double2 vvp = ld2(vvc[o + nc]);  // vv at u level q+1
-    double2 du;
-    const int ibs = ibslot_v ? ibslot_v[q] : -1;
-    if (ibs < 0) {
-      const double a = d0[q], dg = (k2x + k2z) + d1[q], cc = d2[q];
-      double2 L;
-      L.x = (a * vm1.x + dg * v0.x) + cc * vp1.x; L.y = (a * vm1.y + dg * v0.y) + cc * vp1.y;
-      const double C3 = -dR * g.dd * g.thv[q];
-      const double2 pp = p[(size_t)q * nc + c], pm = p[(size_t)(q - 1) * nc + c];
-      const double2 no = Nu2[o];
-      du.x = (C1 * L.x + C2 * no.x) + C3 * (pp.x - pm.x);
-      du.y = (C1 * L.y + C2 * no.y) + C3 * (pp.y - pm.y);
-      const double th = g.thv[q];
-      const double2 x2 = ld2(N2xz[o]);
-      double2 n2;
-      n2.x = x2.x + (vvp.x - vvq.x) * th * g.dd; n2.y = x2.y + (vvp.y - vvq.y) * th * g.dd;
-      Nu2[o] = n2;
-      du.x = du.x + G * n2.x; du.y = du.y + G * n2.y;
+  const int fy = NF == 2 || V ? 0 : (int)blockIdx.y;
+  const double uk = unit * (g.k2x[kx] + g.k2z[r]);
+  const double aR = g.aRK[kRK - 1], bR = g.bRK[kRK - 1];
+  const double c2 = -dt * g.cRK[kRK - 1], cg = -dt * g.gRK[kRK - 1], cp = -dt * g.dRK[kRK - 1];
+  const double mp = (!V && c == 0) ? cp * sc->mpgx : 0.0;  // u only, real part
+  const double gw0 = V ? 0.0 : g.gw[bd][0], gw1 = V ? 0.0 : g.gw[bd][1];
+  const size_t ls = (size_t)nc * 2, ci = (size_t)c * 2 + part, co = (size_t)c * 2 + (NP == 1 ? part ^ 1 : 0);
+  double *u[NF], *No[NF];
+  const double *X[NF], *F[NF];
+  double ck[NF];  // -dt dRK k of the field's gradient
+  int fd[NF];     // field in duib
+#pragma unroll
+  for (int f = 0; f < NF; ++f) {
+    const bool w = f == 1 || fy == 1;
+    u[f] = (w ? a.u[1] : a.u[0]) + ci; No[f] = (w ? a.Nu[1] : a.Nu[0]) + ci;
+    X[f] = (w ? a.X[1] : a.X[0]) + ci; F[f] = (w ? a.F[1] : a.F[0]) + ci;
+    ck[f] = V ? 0.0 : cp * (f + fy ? g.k1z[r] : g.k1x[kx]);
+    fd[f] = V ? 1 : (f + fy ? 2 : 0);
+  }
+  double *a3 = a.a3s + (size_t)fy * (NP == 1 ? 2 : 1) * nlev * nc + (size_t)part * nlev * nc + c;
+#define RS(s_, k_) ring[((s_) * NE + (k_)) * NT + threadIdx.x]
+  // slot of level q: the fields one level up, p, Nu, X, flux (v: v one level up, p at q, Nu, X, vv one up)
+  auto fetch = [&](int q) {
+    const int s_ = (q - qlo - 1) % NS;
+    const size_t o = (size_t)q * ls;
+    if (V) {
+      cpa_part(&RS(s_, 0), u[0] + o + ls); cpa_part(&RS(s_, 1), a.p + o + ci);
+      cpa_part(&RS(s_, 2), No[0] + o); cpa_part(&RS(s_, 3), X[0] + o); cpa_part(&RS(s_, 4), F[0] + o + ls);
     } else {
-      du = duib[((size_t)ibs * 3 + 1) * nc + c];
+      cpa_part(&RS(s_, 0), a.p + o - ls + co);
+#pragma unroll
+      for (int f = 0; f < NF; ++f) {
+        cpa_part(&RS(s_, 1 + 4 * f), u[f] + o + ls); cpa_part(&RS(s_, 2 + 4 * f), No[f] + o);
+        cpa_part(&RS(s_, 3 + 4 * f), X[f] + o); cpa_part(&RS(s_, 4 + 4 * f), F[f] + o);
+      }
     }
-    double2 rhs;
-    rhs.x = v0.x + dt * du.x; rhs.y = v0.y + dt * du.y;
-    const double a1 = -beta * d0[q];
-    const double a2 = 1.0 - beta * ((d1[q] + k2x) + k2z);
-    const double a3p = a3raw * a2p;
-    a3s[(size_t)(q - 1) * nc + c] = a3p;
-    a2p = 1.0 / (a2 - a1 * a3p);
-    y.x = (rhs.x - a1 * y.x) * a2p; y.y = (rhs.y - a1 * y.y) * a2p;
-    u2[o] = y;
-    a3raw = -beta * d2[q];
-    vm1 = v0; v0 = vp1; vvq = vvp;
+  };
+  T um[NF], u0[NF], fl[NF], y[NF], pm;
+  const size_t e0 = (size_t)qlo * ls;
+#pragma unroll
+  for (int f = 0; f < NF; ++f) {
+    um[f] = *reinterpret_cast<const T *>(u[f] + e0);
+    u0[f] = *reinterpret_cast<const T *>(u[f] + e0 + ls);
+    fl[f] = *reinterpret_cast<const T *>(F[f] + e0 + (V ? ls : 0));
   }
-  {
-    const int q = qhi;
-    const double a3p = a3raw * a2p;
-    a3s[(size_t)(q - 1) * nc + c] = a3p;
-    a2p = 1.0 / (1.0 - 0.0 * a3p);
-    y.x = (0.0 - 0.0 * y.x) * a2p; y.y = (0.0 - 0.0 * y.y) * a2p;
-    u2[(size_t)q * nc + c] = y;
+  if (V) pm = *reinterpret_cast<const T *>(a.p + e0 + ci);
+#pragma unroll
+  for (int s_ = 0; s_ < D; ++s_) {
+    if (qlo + 1 + s_ <= qhi - 1) fetch(qlo + 1 + s_);
+    cpa_commit();
   }
-  double2 x = y;
+  double a3raw = gw0, a2p = 1.0;  // first row: [1, gw(b,1)], rhs 0
+#pragma unroll
+  for (int f = 0; f < NF; ++f) {
+#pragma unroll
+    for (int s = 0; s < NP; ++s) comp(y[f], s) = 0.0;
+    *reinterpret_cast<T *>(u[f] + e0) = y[f];
+  }
+  for (int q = qlo + 1; q <= qhi - 1; ++q) {
+    cpa_wait<D - 1>();
+    const int s_ = (q - qlo - 1) % NS;
+    T w[NE];
+#pragma unroll
+    for (int k = 0; k < NE; ++k) w[k] = RS(s_, k);
+    if (q + D <= qhi - 1) fetch(q + D);
+    cpa_commit();
+    const double l1 = t1[q], l2 = t2[q] + uk, l3 = t3[q], th = tth[q], a1 = bR * l1;
+    const int ibs = tib[q];
+    const double a3p = a3raw * a2p;
+    a3[(size_t)(q - 1) * nc] = a3p;
+    a2p = 1.0 / ((1.0 + bR * l2) - a1 * a3p);
+    const size_t o = (size_t)q * ls;
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      T &up = w[V ? 0 : 1 + 4 * f];
+      T rhs;
+      if (ibs < 0) {
+        T &no = w[2 + 4 * f], &x = w[3 + 4 * f], &fq = w[4 + 4 * f];
+        T n;
+#pragma unroll
+        for (int s = 0; s < NP; ++s) {
+          const double t = l1 * comp(um[f], s) + (l2 * comp(u0[f], s) + l3 * comp(up, s));
+          const double nn = comp(x, s) + (comp(fq, s) - comp(fl[f], s)) * th;
+          comp(n, s) = nn;
+          double v = c2 * comp(no, s) - aR * t;  // the increment first: u's rounding enters once
+          v += cg * nn;
+          if (V) {
+            v += (cp * th) * (comp(w[1], s) - comp(pm, s));
+          } else {  // i k p: the other part, with its sign
+            const double pk = NP == 2 ? comp(w[0], s ^ 1) : comp(w[0], 0);
+            const bool re = NP == 2 ? s == 0 : part == 0;
+            v += (re ? -ck[f] : ck[f]) * pk;
+            if (f + fy == 0 && re) v += mp;
+          }
+          comp(rhs, s) = comp(u0[f], s) + v;
+        }
+        *reinterpret_cast<T *>(No[f] + o) = n;
+      } else {
+        T di = *reinterpret_cast<const T *>(a.duib + ((size_t)ibs * 3 + fd[f]) * ls + ci);
+#pragma unroll
+        for (int s = 0; s < NP; ++s) comp(rhs, s) = comp(u0[f], s) + dt * comp(di, s);
+      }
+#pragma unroll
+      for (int s = 0; s < NP; ++s) comp(y[f], s) = (comp(rhs, s) - a1 * comp(y[f], s)) * a2p;
+      *reinterpret_cast<T *>(u[f] + o) = y[f];
+      um[f] = u0[f]; u0[f] = up; fl[f] = w[4 + 4 * f];
+    }
+    if (V) pm = w[1];
+    a3raw = bR * l3;
+  }
+  cpa_wait<0>();
+  {  // last row: [gw(b,2), 1], rhs 0
+    const double a3p = a3raw * a2p;
+    a3[(size_t)(qhi - 1) * nc] = a3p;
+    a2p = 1.0 / (1.0 - gw1 * a3p);
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+#pragma unroll
+      for (int s = 0; s < NP; ++s) comp(y[f], s) = (0.0 - gw1 * comp(y[f], s)) * a2p;
+      *reinterpret_cast<T *>(u[f] + (size_t)qhi * ls) = y[f];
+    }
+  }
+  __threadfence();  // the copies below read what this thread stored above
+  double *ra = reinterpret_cast<double *>(ring + (size_t)NF * NS * NT);  // factors beside the fields' slots
+  auto fetch_b = [&](int q) {
+    const int s_ = (qhi - 1 - q) % NS;
+#pragma unroll
+    for (int f = 0; f < NF; ++f) cpa_part(&ring[(s_ * NF + f) * NT + threadIdx.x], u[f] + (size_t)q * ls);
+    cpa8(&ra[s_ * NT + threadIdx.x], a3 + (size_t)q * nc);
+  };
+#pragma unroll
+  for (int s_ = 0; s_ < D; ++s_) {
+    if (qhi - 1 - s_ >= qlo) fetch_b(qhi - 1 - s_);
+    cpa_commit();
+  }
   for (int q = qhi - 1; q >= qlo; --q) {
-    const size_t o = (size_t)q * nc + c;
-    const double a3p = a3s[o];
-    const double2 yy = u2[o];
-    x.x = yy.x - a3p * x.x; x.y = yy.y - a3p * x.y;
-    u2[o] = x;
+    cpa_wait<D - 1>();
+    const int s_ = (qhi - 1 - q) % NS;
+    T yy[NF];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) yy[f] = ring[(s_ * NF + f) * NT + threadIdx.x];
+    const double a3p = ra[s_ * NT + threadIdx.x];
+    if (q - D >= qlo) fetch_b(q - D);
+    cpa_commit();
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+#pragma unroll
+      for (int s = 0; s < NP; ++s) comp(y[f], s) = comp(yy[f], s) - a3p * comp(y[f], s);
+      *reinterpret_cast<T *>(u[f] + (size_t)q * ls) = y[f];
+    }
   }
+  cpa_wait<0>();
+#undef RS
 }
 
 // ============================================================================
@@ -601,17 +659,6 @@ __global__ void __launch_bounds__(512) k_helm00_pcr(double *__restrict__ u1, dou
   for (int i = threadIdx.x; i < n; i += blockDim.x) u[(qlo + i) * ls + part] = D[i] / B[i];
 }
 
-// cp.async copies from global to shared memory (8 and 4 bytes), their commit groups and waits
-__device__ __forceinline__ void cpa8(void *dst, const void *src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cpa4(void *dst, const void *src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cpa_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cpa_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 // ============================================================================
 // Mixed-form solves with one lane per (column, real/imaginary part): the matrix
