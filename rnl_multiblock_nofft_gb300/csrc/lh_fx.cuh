@@ -91,17 +91,13 @@ __host__ __device__ __forceinline__ fx2 fx_in2(double2 z, const FxScale &s) {
   r.y = fx_in(z.y, s.k0);
   return r;
 }
-// v * 2^-S rounded to nearest. Two FP64 additions (the FP64 pipe has nothing else to do) in
-// place of a count-leading-zeros and shift sequence on the busy integer pipe.
+// v * 2^-S rounded to nearest. The hardware conversion counts as one operation of the FP64 pipe
+// (two FP64 additions on split halves measured as two); the scaling is an exponent add.
 __host__ __device__ __forceinline__ double fx_out(long long v, int S) {
 #ifdef __CUDA_ARCH__
-  const int hi = (int)(v >> 32);
-  const double h = __dadd_rn(__hiloint2double(0x45300000, hi ^ (int)0x80000000), -0x1.00000801p+84);
-  double r = __dadd_rn(h, __hiloint2double(0x43300000, (int)v));
-  if ((unsigned)(S + 900) <= 1900u) {
-    if (v != 0) r = __hiloint2double(__double2hiint(r) - (S << 20), __double2loint(r));
-    return r;
-  }
+  const double r = __ll2double_rn(v);
+  if ((unsigned)(S + 900) <= 1900u)
+    return v != 0 ? __hiloint2double(__double2hiint(r) - (S << 20), __double2loint(r)) : r;
   if (S < FX_NAN / 2) return __longlong_as_double(0x7ff8000000000000ll);
   return scalbn(r, -S);
 #else
@@ -299,16 +295,17 @@ template <int N, int NL, bool IL>
 __host__ __device__ __forceinline__ int fx_at(int line, int e) { return IL ? e * NL + line : line * N + e; }
 
 // One stage over NL lines. ld(line, e) gives input e of a line, st(line, e, v) takes output e,
-// all(line, v, R) sees a butterfly's outputs first. Inputs t in [Z0, Z1) are zero and not read,
+// all(line, v, R) sees a butterfly's outputs first; nl: lines in use (IL = false). Inputs t in [Z0, Z1) are zero and not read,
 // outputs t in [W0, W1) are not stored; XE (x lines: modes -N/3 .. N/3 are kept): of t = Z0 and
 // t = W0 the element j = 0 is kept.
 #pragma nv_exec_check_disable
 template <int N, int NL, bool IL, bool INV, int ST, int Z0, int Z1, int W0, int W1, bool XE, class LD, class SF, class AL>
-__host__ __device__ __forceinline__ void fx_stage(int tid, int nthr, const int4 *__restrict__ tw, LD ld, SF st, AL all) {
+__host__ __device__ __forceinline__ void fx_stage(int tid, int nthr, const int4 *__restrict__ tw, LD ld, SF st, AL all,
+                                                  int nl = NL) {
   constexpr int R = fx_radix<N, INV>(ST);
   constexpr int Ns = ST == 0 ? 1 : ST == 1 ? fx_radix<N, INV>(0) : fx_radix<N, INV>(0) * fx_radix<N, INV>(1);
   constexpr int nb = N / R, step = N / (Ns * R);
-  for (int idx = tid; idx < nb * NL; idx += nthr) {
+  for (int idx = tid; idx < nb * nl; idx += nthr) {
     int line, j;
     if (IL) { j = idx / NL; line = idx - j * NL; }
     else { line = idx / nb; j = idx - line * nb; }
@@ -344,21 +341,21 @@ struct FxNone { __host__ __device__ void operator()(int, const fx2 *, int) const
 // through b1 (after stage 0) and b0 (after stage 1). ld may read b0; st may write the
 // buffer the last stage does not read: b1 (three stages) or b0 (two).
 template <int N, int NL, bool IL, bool INV, int Z0, int Z1, int W0, int W1, bool XE, class LD, class SF, class AL = FxNone>
-__device__ __forceinline__ void fx_fft(fx2 *b0, fx2 *b1, const int4 *__restrict__ tw, LD ld, SF st, AL all = AL()) {
+__device__ __forceinline__ void fx_fft(fx2 *b0, fx2 *b1, const int4 *__restrict__ tw, LD ld, SF st, AL all = AL(), int nl = NL) {
   const int tid = threadIdx.x, nthr = blockDim.x;
   fx_stage<N, NL, IL, INV, 0, Z0, Z1, 0, 0, XE>(tid, nthr, tw, ld,
-      [&](int line, int e, fx2 v) { b1[fx_swz(fx_at<N, NL, IL>(line, e))] = v; }, FxNone());
+      [&](int line, int e, fx2 v) { b1[fx_swz(fx_at<N, NL, IL>(line, e))] = v; }, FxNone(), nl);
   __syncthreads();
   if constexpr (fx_stages(N) == 3) {
     fx_stage<N, NL, IL, INV, 1, 0, 0, 0, 0, false>(tid, nthr, tw,
         [&](int line, int e) { return b1[fx_swz(fx_at<N, NL, IL>(line, e))]; },
-        [&](int line, int e, fx2 v) { b0[fx_swz(fx_at<N, NL, IL>(line, e))] = v; }, FxNone());
+        [&](int line, int e, fx2 v) { b0[fx_swz(fx_at<N, NL, IL>(line, e))] = v; }, FxNone(), nl);
     __syncthreads();
     fx_stage<N, NL, IL, INV, 2, 0, 0, W0, W1, XE>(tid, nthr, tw,
-        [&](int line, int e) { return b0[fx_swz(fx_at<N, NL, IL>(line, e))]; }, st, all);
+        [&](int line, int e) { return b0[fx_swz(fx_at<N, NL, IL>(line, e))]; }, st, all, nl);
   } else {
     fx_stage<N, NL, IL, INV, 1, 0, 0, W0, W1, XE>(tid, nthr, tw,
-        [&](int line, int e) { return b1[fx_swz(fx_at<N, NL, IL>(line, e))]; }, st, all);
+        [&](int line, int e) { return b1[fx_swz(fx_at<N, NL, IL>(line, e))]; }, st, all, nl);
   }
 }
 #endif

@@ -6,9 +6,10 @@
 //
 // Measured at 256 x 256 x 301 with posts (transforms of 384), ms per step (three launches),
 // against the FP64 Stockham passes that they replaced (FP64 pipe 85 % busy, DRAM 2-5 %):
-//   inverse z 18.52 -> 6.20, x 62.94 -> 16.85, forward z 19.01 -> 7.39, immersed-boundary
-//   x round trip 6.58 -> 2.00, its z transforms 1.95 -> 0.57 and 2.04 -> 0.61; the whole
-//   step 123.4 -> 46.2. The integer pipe bounds them now.
+//   inverse z 18.52 -> 4.98, x 62.94 -> 15.37, forward z 19.01 -> 6.50, immersed-boundary
+//   x round trip 6.58 -> 1.76, its z transforms 1.95 -> 0.51 and 2.04 -> 0.54; the whole
+//   step 123.4 -> 39.2 (6.20, 16.85, 7.39 and 43.0 with two FP64 additions per converted
+//   result, which kept the FP64 pipe 57-74 % busy). Instruction issue bounds them now.
 #pragma once
 #include "lh_fx.cuh"
 #include "lh_kernels.cuh"
@@ -436,14 +437,16 @@ template <int N, int NL> __host__ __device__ constexpr int fx_xslots() {
 // transform. The products are formed from the integer fields, normalised by each field's
 // largest value on the line, as the forward transform's first stage reads them.
 // ============================================================================
-template <int N, int NPR, int PB>
-__device__ __forceinline__ void fx_xpass_forward(const fx2 *res, fx2 *oth, fx2 *rsv, const int *fl, const int *fS, int *sP,
+// Products uu, uw, vv, ww (u level) or uv, wv (v level) of the fields' lines f * PB + pb in res and
+// their forward transforms, lines p * PB + pb in res (two stages) or oth (three). One code for
+// both kinds of level: the kernel's code has to stay in the instruction cache.
+template <int N, int PB>
+__device__ __forceinline__ void fx_xpass_forward(bool isU, fx2 *res, fx2 *oth, const int *fl, const int *fS, int *sP,
                                                  const int4 *__restrict__ tw) {
-  // operand lines of product p: uu, uw, vv, ww (u level); uv, wv (v level)
   constexpr int RL = fx_radix<N, false>(fx_stages(N) - 1);
   constexpr int DROP = fx_drop<N>();
-  auto fa = [](int p) { return NPR == 4 ? (p == 0 ? 0 : p == 1 ? 0 : p == 2 ? 1 : 2) : (p == 0 ? 0 : 2); };
-  auto fb = [](int p) { return NPR == 4 ? (p == 0 ? 0 : p == 1 ? 2 : p == 2 ? 1 : 2) : 1; };
+  auto fa = [&](int p) { return isU ? (p > 0 ? p - 1 : 0) : 2 * p; };
+  auto fb = [&](int p) { return isU ? (p == 0 ? 0 : p == 2 ? 1 : 2) : 1; };
   auto shift = [](fx2 v, int l) {
     const int a = l > 0 ? l : 0, b = l < 0 ? -l : 0;
     fx2 r;
@@ -451,7 +454,8 @@ __device__ __forceinline__ void fx_xpass_forward(const fx2 *res, fx2 *oth, fx2 *
     r.y = (long long)((unsigned long long)v.y << a) >> b;
     return r;
   };
-  if (threadIdx.x < NPR * PB) {
+  const int nl = (isU ? 4 : 2) * PB;
+  if ((int)threadIdx.x < nl) {
     const int p = threadIdx.x / PB, pb = threadIdx.x - p * PB, a = fa(p) * PB + pb, b = fb(p) * PB + pb;
     sP[threadIdx.x] = (fS[a] == FX_NAN || fS[b] == FX_NAN) ? FX_NAN : fS[a] + fl[a] + fS[b] + fl[b] - 64 - DROP;
   }
@@ -463,10 +467,10 @@ __device__ __forceinline__ void fx_xpass_forward(const fx2 *res, fx2 *oth, fx2 *
     r.y = fx_mul(x.y, y.y);
     return r;
   };
-  fx2 *last = fx_stages(N) == 3 ? oth : rsv;
-  // stage 0 reads res and writes oth, stage 1 writes res' buffer, the last stage writes `last`
-  fx_fft<N, NPR * PB, false, false, 0, 0, RL / 3, 2 * RL / 3, true>(
-      rsv, oth, tw, ld, [&](int line, int e, fx2 v) { last[line * N + e] = v; });
+  fx2 *last = fx_stages(N) == 3 ? oth : res;
+  // stage 0 reads res and writes oth, stage 1 writes res, the last stage writes `last`
+  fx_fft<N, 4 * PB, false, false, 0, 0, RL / 3, 2 * RL / 3, true>(
+      res, oth, tw, ld, [&](int line, int e, fx2 v) { last[line * N + e] = v; }, FxNone(), nl);
   __syncthreads();
 }
 
@@ -555,9 +559,7 @@ __global__ void __launch_bounds__(fx_xt(N)) k_xpass_fx(const double2 *__restrict
       else atomic_max_pos(&sc->u2m, m0);
     }
   }
-  // forward: three stages end in oth, two in res' buffer
-  if (isU) fx_xpass_forward<N, 4, PB>(res, oth, res, fl, fS, sP, tw);
-  else fx_xpass_forward<N, 2, PB>(res, oth, res, fl, fS, sP, tw);
+  fx_xpass_forward<N, PB>(isU, res, oth, fl, fS, sP, tw);
   const fx2 *pres = fx_stages(N) == 3 ? oth : res;
   const int nprod = isU ? 4 : 2;
   const int pbase = isU ? slot_i * 4 : g.nuI * 4 + (slot_i - g.nuI) * 2;
