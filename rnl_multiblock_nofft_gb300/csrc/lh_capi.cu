@@ -32,7 +32,7 @@ struct lh_handle {
   size_t vsz;  // bytes of one complex value in the transforms
   cudaStream_t st;
   cudaStream_t st2;            // side stream: mean-flow correction overlapped with the v solve
-  cudaEvent_t ev_fork, ev_join;
+  cudaEvent_t ev_fork, ev_join, ev_mf;
   // device buffers
   double2 *u1, *u2, *u3, *p, *psi;
   void *Nu1, *Nu2, *Nu3;  // nonlinear term of the last substep, transform precision
@@ -546,7 +546,8 @@ extern "C" int lh_create(const lh_config *cfg, lh_handle **out) {
   if (cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&h->st2, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming) != cudaSuccess) {
+      cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&h->ev_mf, cudaEventDisableTiming) != cudaSuccess) {
     int rc = fail(h, LH_ECUDA, "cudaStreamCreate/cudaEventCreate"); lh_destroy(h); return rc;
   }
   {  // views: slot tables, capture slots of view 0, twiddles; solve segments; band columns
@@ -716,6 +717,7 @@ extern "C" int lh_destroy(lh_handle *h) {
   if (h->st_out) cudaStreamDestroy(h->st_out);
   if (h->ev_fork) cudaEventDestroy(h->ev_fork);
   if (h->ev_join) cudaEventDestroy(h->ev_join);
+  if (h->ev_mf) cudaEventDestroy(h->ev_mf);
   if (h->st2) cudaStreamDestroy(h->st2);
   if (h->st) cudaStreamDestroy(h->st);
   delete h;
@@ -1239,20 +1241,18 @@ static int phys_to_spec(lh_handle *h, const double *phys, double2 *spec, int npl
 
 static const void *fp64_tw(lh_handle *h, bool x) { return x ? h->twx64 : h->twz64; }
 
-// flowrate_corr after solveU_W, on the side stream (joined before solveP); on the
-// main stream when kernels are being timed one by one
-// flowrate_corr on the main stream, after the u solve (constant flow rate only)
-static int meanflow(lh_handle *h, int kRK) {
+// flowrate_corr after the u solve of mode (0,0) (constant flow rate only)
+static int meanflow(lh_handle *h, int kRK, cudaStream_t st) {
   const Geo &g = h->g;
   if (g.flag_ctpress != 0) return LH_OK;
   const size_t pcr = 8 * sizeof(double) * (size_t)(g.nn + 3);
   if (pcr <= 96 * 1024) {  // parallel cyclic reduction in one block
-    KL("k_meanflow", k_meanflow_pcr<<<1, 512, pcr, h->st>>>(h->u1, g, h->sc, kRK));
+    KL("k_meanflow", k_meanflow_pcr<<<1, 512, pcr, st>>>(h->u1, g, h->sc, kRK));
     return LH_OK;
   }
   const size_t mb = 6 * sizeof(double) * (size_t)(g.nn + 3);
   const int sm = mb <= 48 * 1024 ? 1 : 0;
-  KL("k_meanflow", k_meanflow<<<1, 256, sm ? mb : 0, h->st>>>(h->u1, g, h->sc, kRK, h->mfw, sm));
+  KL("k_meanflow", k_meanflow<<<1, 256, sm ? mb : 0, st>>>(h->u1, g, h->sc, kRK, h->mfw, sm));
   return LH_OK;
 }
 
@@ -1325,9 +1325,10 @@ static int substep_launches_t(lh_handle *h, int kRK) {
   // mean-flow correction (which follows u) run on the main stream; each solve has its
   // own scratch. In the mixed form mode (0,0) is solved in FP64 by its own kernel on the
   // side stream after v (the other solves skip column 0), overlapping the longer u/w solve;
-  // the mean-flow correction, which reads u(0,0), follows the join. (Sequential on the main
-  // stream while per-kernel times are profiled.)
+  // the mean-flow correction, which changes u(0,0) alone, follows it there. (Sequential on the
+  // main stream while per-kernel times are profiled.)
   const bool fork = !h->prof;
+  const bool split = g.nvc < LH_PRESS_SPLIT_COLS;
   cudaStream_t sv = fork ? h->st2 : h->st;
   if (fork) {
     CK(cudaEventRecord(h->ev_fork, h->st));
@@ -1363,6 +1364,10 @@ static int substep_launches_t(lh_handle *h, int kRK) {
                        g, h->sc, kRK, h->a3s));
   }
   if (fork) CK(cudaEventRecord(h->ev_join, h->st2));
+  if (mixed00 && fork && split) {  // u(0,0) is solved: its flow-rate correction, beside the u/w solve
+    if ((rc = meanflow(h, kRK, sv))) return rc;
+    CK(cudaEventRecord(h->ev_mf, h->st2));
+  }
   if (h->prec == LH_PREC_FP64) {
     KL("k_helm_uw", launch_helm64_uw(h, kRK));
   } else {
@@ -1383,11 +1388,31 @@ static int substep_launches_t(lh_handle *h, int kRK) {
     }
   }
   if (fork) CK(cudaStreamWaitEvent(h->st, h->ev_join, 0));
-  if ((rc = meanflow(h, kRK))) return rc;
+  // otherwise the mean-flow correction follows the join: beside the pressure's right-hand side and
+  // sweep where these are launches of their own (they read u(0,0) times k = 0), else before. (Large
+  // channels fill the GPU: beside their solves it cost a step 0.8 %.)
+  if (!(mixed00 && fork && split)) {
+    const bool beside = fork && split;
+    if (beside) {
+      CK(cudaEventRecord(h->ev_fork, h->st));
+      CK(cudaStreamWaitEvent(h->st2, h->ev_fork, 0));
+    }
+    if ((rc = meanflow(h, kRK, beside ? h->st2 : h->st))) return rc;
+    if (beside) CK(cudaEventRecord(h->ev_mf, h->st2));
+  }
+  const bool mf_side = g.flag_ctpress == 0 && fork && split;
   const int need_div = (kRK == 3) ? 1 : 0;
   if (need_div) KL("k_reset_err", k_reset_err<<<1, 32, 0, h->st>>>(h->sc));
   const int nbp2 = (2 * g.nvc + h->tb_p - 1) / h->tb_p;
-  {  // the pressure step with its y-columns staged pf_p levels ahead (k_press3)
+  if (split) {  // the corrections wait for the mean-flow kernel, which may run beside the sweep
+    const dim3 ge((g.nvc + 127) / 128, (g.np + LH_PL - 1) / LH_PL);
+    double2 *vlow = need_div ? (double2 *)h->A : nullptr;  // (the transforms' scratch is free here)
+    KL("k_press_rhs", k_press_rhs<<<ge, 128, 0, h->st>>>(h->u1, h->u2, h->u3, h->psi, vlow, g, h->sc, kRK));
+    KL("k_press", k_press_sweep<<<(2 * g.nvc + 31) / 32, 32, 0, h->st>>>((double *)h->psi, h->dg1, h->dg2, h->dg3, g));
+    if (mf_side) CK(cudaStreamWaitEvent(h->st, h->ev_mf, 0));
+    if (need_div) KL("k_press_corr", k_press_corr<true><<<ge, 128, 0, h->st>>>(h->u1, h->u2, h->u3, h->p, h->psi, vlow, g, h->sc, kRK));
+    else KL("k_press_corr", k_press_corr<false><<<ge, 128, 0, h->st>>>(h->u1, h->u2, h->u3, h->p, h->psi, vlow, g, h->sc, kRK));
+  } else {  // the pressure step with its y-columns staged pf_p levels ahead (k_press3)
     const size_t sm = press_smem(g, h->pf_p, h->tb_p);
     double *U1 = (double *)h->u1, *U2 = (double *)h->u2, *U3 = (double *)h->u3, *P = (double *)h->p;
     double *PS = (double *)h->psi;

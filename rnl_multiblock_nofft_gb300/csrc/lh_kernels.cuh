@@ -13,7 +13,7 @@
 //   k_helm_uw   : RHS0_u1/u3 + der_yu_h + du += -gRK N + solveU_W, one thread per column
 //   k_helm_v    : RHS0_u2 + der_yv_h + du += -gRK N + solveV
 //   k_meanflow  : flowrate_corr on mode (0,0) (constant flow rate)
-//   k_press2    : divergence + solveP (LUsolP with the stored factors, k_build_dg) + v_corr
+//   k_press3 (k_press2), or k_press_rhs, k_press_sweep, k_press_corr : divergence + solveP (LUsolP with the stored factors, k_build_dg) + v_corr
 //                 + divergence of the corrected field in the third substep (max |div| -> err)
 //   k_ib_du(_mx), k_spec_zinv(_fx, 2), k_ib_xforce(_fx), k_zfwd_spec(_fx, 2) : immersed-boundary
 //                 forcing of du (imm_bounds_u/v, FOU3D.f90:806-998) when the geometry has posts
@@ -264,6 +264,10 @@ __device__ __forceinline__ void cpa8(void *dst, const void *src) {
 __device__ __forceinline__ void cpa4(void *dst, const void *src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
+}
+// the same on a 32-bit shared address
+__device__ __forceinline__ void cpa8s(unsigned dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cpa_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cpa_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
@@ -1310,10 +1314,17 @@ __global__ void __launch_bounds__(512) k_meanflow_pcr(double2 *__restrict__ u1, 
     ur[j] = u1[(size_t)(j + dny) * nc].x;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double Qx1 = 0.0, Qx0 = 0.0;
-    for (int j = 1; j <= nn + 1; ++j) Qx1 = Qx1 + dy[j] * D[j];
+  if (threadIdx.x == 32) {  // (a warp each: two serial sums side by side)
+    double Qx0 = 0.0;
     for (int j = 1; j <= nn + 1; ++j) Qx0 = Qx0 + dy[j] * ur[j];
+    gg_sh = Qx0;
+  }
+  double Qx1 = 0.0;
+  if (threadIdx.x == 0)
+    for (int j = 1; j <= nn + 1; ++j) Qx1 = Qx1 + dy[j] * D[j];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const double Qx0 = gg_sh;
     const double gg = (sc->QxT - Qx0) / Qx1;
     sc->mpgx = sc->mpgx + gg;
     sc->dgx = gg;
@@ -1717,6 +1728,231 @@ __global__ void __launch_bounds__(NTHR) k_press3(double *__restrict__ u1, double
 #undef RS
   dmax = warp_max_bits(dmax);
   if ((threadIdx.x & 31) == 0) atomicMax(&sc->errbits, dmax);
+}
+
+// ============================================================================
+// The pressure step of channels below LH_PRESS_SPLIT_COLS columns in three launches. An FP64 warp
+// instruction holds its scheduler's half lane a clock for 64 cycles, so k_press3's sweep, which
+// also forms its right-hand side and applies its result (12 FP64 instructions a level), is a
+// chain of 768 cycles a level however few columns there are. Here the right-hand side and the
+// corrections are element-wise over (column, chunk of levels), and the sweep keeps the
+// recurrences: two dependent operations a level up, one down. The same operations in the same
+// order per element, so the same results bit for bit, and no more FP64 operations; but psi
+// crosses memory three more times (3.7 instead of 2.9 GB at 256 x 256 x 301), so larger channels
+// keep the fused sweep. us a launch, fused -> the three launches together: 32 x 32 x 153 (544
+// columns) 143 -> 59, 128 x 96 x 201 (6240) 190 -> 127. us a step, mixed form alone / among others:
+// 128 x 128 x 201 (8320) 1784 / 1330 -> 1555 / 1263, 192 x 128 x 201 (12416) 2368 / 2004 -> 2184 /
+// 2003, 192 x 192 x 201 (18624) 3025 / 2936 -> 3100 / 3038.
+// ============================================================================
+#define LH_PRESS_SPLIT_COLS 16384
+#define LH_PL 8  // levels of a thread of the element-wise kernels (rolling v, psi)
+// a b + c d + t dv with the roundings of k_press3's compiled expression (the fused operations are
+// written out throughout, so that both routes of the pressure step agree bit for bit)
+__device__ __forceinline__ double press_div(double a, double b, double c, double d, double t, double dv) {
+  return __fma_rn(t, dv, __fma_rn(a, b, __dmul_rn(c, d)));
+}
+// psi = dti/(a+b) div: thread = (column segment, chunk), both parts; vlow (third substep): the face
+// below each chunk, [chunk][segment], for the corrections' divergence
+__global__ void __launch_bounds__(128) k_press_rhs(const double2 *__restrict__ u1, const double2 *__restrict__ u2,
+                                                   const double2 *__restrict__ u3, double2 *__restrict__ psi,
+                                                   double2 *__restrict__ vlow, Geo g, const DevScalars *__restrict__ sc,
+                                                   int kRK) {
+  const int vc = blockIdx.x * 128 + threadIdx.x;
+  if (vc >= g.nvc) return;
+  int c, bd;
+  vcol_of(g, vc, c, bd);
+  const int plo = g.bq[bd][4], phi = g.bq[bd][5];
+  const int q0 = plo + blockIdx.y * LH_PL;
+  if (q0 > phi) return;
+  const int nc = g.ncol, r = c / g.N1h, kx = c - r * g.N1h;
+  const double dtirk = sc->dti / (g.aRK[kRK - 1] + g.bRK[kRK - 1]);
+  const double dkx = dtirk * g.k1x[kx], dkz = dtirk * g.k1z[r];
+  double2 vm = u2[(size_t)q0 * nc + c];
+  if (vlow) vlow[(size_t)blockIdx.y * g.nvc + vc] = vm;
+#pragma unroll
+  for (int i = 0; i < LH_PL; ++i) {
+    const int qp = q0 + i;
+    if (qp > phi) break;
+    const size_t e = (size_t)(qp + 1) * nc + c;
+    const double2 a = u1[e], w = u3[e], v = u2[e];
+    const double th = dtirk * g.thud[qp + 1];
+    double2 rhs;
+    rhs.x = press_div(-dkx, a.y, -dkz, w.y, th, v.x - vm.x);
+    rhs.y = press_div(dkx, a.x, dkz, w.x, th, v.y - vm.y);
+    if (qp == plo && c == 0 && bd == 1) rhs = make_double2(0.0, 0.0);
+    psi[e - nc] = rhs;
+    vm = v;
+  }
+}
+
+// LUsolP in place on psi: lane = (column segment, part), U levels a batch, two batches ahead
+#define LH_PS_U 4
+__host__ __device__ constexpr int press_region() { return 3 * LH_PS_U * 3 | 1; }  // doubles of a thread's ring
+__global__ void __launch_bounds__(32) k_press_sweep(double *__restrict__ psi, const double *__restrict__ dg1,
+                                                    const double *__restrict__ dg2, const double *__restrict__ dg3, Geo g) {
+  constexpr int U = LH_PS_U, BE = 3 * U;
+  __shared__ double ring_all[32 * press_region()];
+  double *ring = ring_all + threadIdx.x * press_region();
+  const unsigned rs = (unsigned)__cvta_generic_to_shared(ring);
+  const int tid = blockIdx.x * 32 + threadIdx.x, vc = tid >> 1, part = tid & 1;
+  if (vc >= g.nvc) return;
+  int c, bd;
+  vcol_of(g, vc, c, bd);
+  const int plo = g.bq[bd][4], phi = g.bq[bd][5];
+  const size_t nc = g.ncol, ls = 2 * nc, ci = 2 * (size_t)c + part;
+  double y = 0.0;
+  {  // forward: a level's right-hand side, dg1, dg2
+    const double *fs = psi + (size_t)plo * ls + ci, *f1 = dg1 + (size_t)plo * nc + c, *f2 = dg2 + (size_t)plo * nc + c;
+    double *ps = psi + (size_t)plo * ls + ci;
+    int left = phi - plo + 1;
+    unsigned dst = rs;
+    auto fetch = [&]() {
+#pragma unroll
+      for (int i = 0; i < U; ++i) {
+        if (left > i) {
+          cpa8s(dst + 24 * i, fs); cpa8s(dst + 24 * i + 8, f1); cpa8s(dst + 24 * i + 16, f2);
+          fs += ls; f1 += nc; f2 += nc;
+        }
+      }
+      left -= U;
+      dst = dst == rs + 8 * 2 * BE ? rs : dst + 8 * BE;
+      cpa_commit();
+    };
+    fetch();
+    fetch();
+    const double *h = ring;
+    bool first = true;
+    for (int n = phi - plo + 1; n > 0; n -= U) {
+      fetch();
+      cpa_wait<2>();
+#pragma unroll
+      for (int i = 0; i < U; ++i) {
+        if (i > 0 && n <= i) break;
+        const double rhs = h[3 * i], A1 = h[3 * i + 1], a2p = h[3 * i + 2];
+        y = (i == 0 && first) ? __dmul_rn(rhs, a2p) : __dmul_rn(__fma_rn(-A1, y, rhs), a2p);
+        *ps = y;
+        ps += ls;
+      }
+      first = false;
+      h = h == ring + 2 * BE ? ring : h + BE;
+    }
+  }
+  cpa_wait<0>();
+  __threadfence();  // the copies below read what this thread stored above
+  {  // backward from the level below the top: a level's y, dg3
+    const double *fs = psi + (size_t)(phi - 1) * ls + ci, *f3 = dg3 + (size_t)(phi - 1) * nc + c;
+    double *ps = psi + (size_t)(phi - 1) * ls + ci;
+    int left = phi - plo;
+    unsigned dst = rs;
+    auto fetch = [&]() {
+#pragma unroll
+      for (int i = 0; i < U; ++i) {
+        if (left > i) {
+          cpa8s(dst + 24 * i, fs); cpa8s(dst + 24 * i + 8, f3);
+          fs -= ls; f3 -= nc;
+        }
+      }
+      left -= U;
+      dst = dst == rs + 8 * 2 * BE ? rs : dst + 8 * BE;
+      cpa_commit();
+    };
+    fetch();
+    fetch();
+    const double *h = ring;
+    for (int n = phi - plo; n > 0; n -= U) {
+      fetch();
+      cpa_wait<2>();
+#pragma unroll
+      for (int i = 0; i < U; ++i) {
+        if (i > 0 && n <= i) break;
+        y = __fma_rn(-h[3 * i + 1], y, h[3 * i]);
+        *ps = y;
+        ps -= ls;
+      }
+      h = h == ring + 2 * BE ? ring : h + BE;
+    }
+  }
+  cpa_wait<0>();
+}
+
+// p += psi, v_corr, ghost rows, v = 0 at the segment's ends: thread = (column segment, chunk)
+template <bool DIV>
+__global__ void __launch_bounds__(128) k_press_corr(double2 *__restrict__ u1, double2 *__restrict__ u2,
+                                                    double2 *__restrict__ u3, double2 *__restrict__ p,
+                                                    const double2 *__restrict__ psi, const double2 *__restrict__ vlow, Geo g,
+                                                    DevScalars *sc, int kRK) {
+  const int vc = blockIdx.x * 128 + threadIdx.x;
+  unsigned long long dmax = 0ull;  // max |div|^2 as bits
+  int c = 0, bd = 1, plo = 0, phi = -1;
+  if (vc < g.nvc) {
+    vcol_of(g, vc, c, bd);
+    plo = g.bq[bd][4];
+    phi = g.bq[bd][5];
+  }
+  const int q0 = plo + blockIdx.y * LH_PL;
+  if (vc < g.nvc && q0 <= phi) {
+    const int nc = g.ncol, r = c / g.N1h, kx = c - r * g.N1h;
+    const int ulo = g.bq[bd][0], uhi = g.bq[bd][1], vlo = g.bq[bd][2], vhi = g.bq[bd][3];
+    const double kxv = g.k1x[kx], kzv = g.k1z[r], dtrk = sc->dt * (g.aRK[kRK - 1] + g.bRK[kRK - 1]);
+    const double kxd = dtrk * kxv, kzd = dtrk * kzv, dtd = dtrk * g.dd;
+    const int q1 = min(q0 + LH_PL, phi + 1);  // levels q0 .. q1 - 1
+    double2 x = psi[(size_t)q0 * nc + c], vm = make_double2(0.0, 0.0);
+    if (DIV) {  // the face below, corrected here too (another thread stores it, hence the copy)
+      vm = vlow[(size_t)blockIdx.y * g.nvc + vc];
+      if (q0 > plo && q0 <= vhi - 1) {
+        const double2 xm = psi[(size_t)(q0 - 1) * nc + c];
+        const double t = dtd * g.thv[q0];
+        vm.x = __fma_rn(-t, x.x - xm.x, vm.x);
+        vm.y = __fma_rn(-t, x.y - xm.y, vm.y);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < LH_PL; ++i) {
+      const int qp = q0 + i, q = qp + 1;
+      if (qp >= q1) break;
+      const size_t e = (size_t)q * nc + c;
+      double2 pq = p[e - nc], a = u1[e], w = u3[e], v = u2[e], xn = x;
+      if (qp < phi) xn = psi[e];
+      pq.x = pq.x + x.x; pq.y = pq.y + x.y;
+      a.x = __fma_rn(kxd, x.y, a.x); a.y = __fma_rn(-kxd, x.x, a.y);
+      w.x = __fma_rn(kzd, x.y, w.x); w.y = __fma_rn(-kzd, x.x, w.y);
+      p[e - nc] = pq;
+      u1[e] = a;
+      u3[e] = w;
+      if (q <= vhi - 1) {
+        const double t = dtd * g.thv[q];
+        v.x = __fma_rn(-t, xn.x - x.x, v.x);
+        v.y = __fma_rn(-t, xn.y - x.y, v.y);
+        u2[e] = v;
+      }
+      if (DIV) {
+        const double t = g.thud[q];
+        const double dx = press_div(-kxv, a.y, -kzv, w.y, t, v.x - vm.x);
+        const double dy = press_div(kxv, a.x, kzv, w.x, t, v.y - vm.y);
+        bits_max(dmax, __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
+        vm = v;
+      }
+      if (qp == plo) {
+        if (bd <= 1) {
+          u1[(size_t)ulo * nc + c] = cscale(a, g.gwbc1);
+          u3[(size_t)ulo * nc + c] = cscale(w, g.gwbc3);
+        }
+        u2[(size_t)vlo * nc + c] = make_double2(0.0, 0.0);
+      }
+      if (qp == phi) {
+        if (bd >= 1) {
+          u1[(size_t)uhi * nc + c] = cscale(a, g.gwbc1);
+          u3[(size_t)uhi * nc + c] = cscale(w, g.gwbc3);
+        }
+        u2[(size_t)vhi * nc + c] = make_double2(0.0, 0.0);
+      }
+      x = xn;
+    }
+  }
+  if (DIV) {
+    dmax = warp_max_bits(dmax);
+    if ((threadIdx.x & 31) == 0) atomicMax(&sc->errbits, dmax);
+  }
 }
 
 __global__ void k_reset_err(DevScalars *sc) {
