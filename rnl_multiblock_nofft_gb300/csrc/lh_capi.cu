@@ -423,7 +423,7 @@ extern "C" int lh_create(const lh_config *cfg, lh_handle **out) {
   ZA(h->N2xz, vs * nv * nc); ZA(h->uvf, vs * nv * nc); ZA(h->wvf, vs * nv * nc);
   // a3s: the FP64 solves' upper factors; in the mixed form the previous nonlinear term of mode
   // (0,0) in FP64 (k_helm00_pcr: 6 x nu doubles; nc >= 8 always)
-  const size_t split = h->prec == LH_PREC_FP64 && g.nvc < LH_H64_SPLIT ? 2 : 1;  // k_helm64<., 1, 1>: factors per field and part
+  const size_t split = h->prec == LH_PREC_FP64 && g.nvc < LH_HELM_SPLIT ? 2 : 1;  // k_helm_sweep64: factors per field and part
   ZA(h->psi, cz * g.np * nc); ZA(h->a3s, split * split * sizeof(double) * nu * nc); ZA(h->a3v, split * sizeof(double) * nv * nc);
   ZA(h->mfw, sizeof(double) * 6 * (size_t)(g.nn + 3));
   h->Abytes = h->Bbytes = 0;
@@ -621,10 +621,9 @@ extern "C" int lh_create(const lh_config *cfg, lh_handle **out) {
     if (smem_optin(&lim) || cudaFuncSetAttribute((const void *)k_press3<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
         cudaFuncSetAttribute((const void *)k_press3<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
         cudaFuncSetAttribute((const void *)k_press3<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
-        cudaFuncSetAttribute((const void *)k_helm64<false, 2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
-        cudaFuncSetAttribute((const void *)k_helm64<false, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
-        cudaFuncSetAttribute((const void *)k_helm64<true, 1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
-        cudaFuncSetAttribute((const void *)k_helm64<true, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
+        cudaFuncSetAttribute((const void *)k_helm_sweep64, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
+        cudaFuncSetAttribute((const void *)k_helm64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
+        cudaFuncSetAttribute((const void *)k_helm64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
         cudaFuncSetAttribute((const void *)k_helm_u_mx3<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
         cudaFuncSetAttribute((const void *)k_helm_u_mx3<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
         cudaFuncSetAttribute((const void *)k_helm_u_mx3<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
@@ -1265,28 +1264,32 @@ static size_t press_smem(const Geo &g, int pf, int tb) {
   return sizeof(double) * (((size_t)g.nu + g.nv + 1) & ~(size_t)1) + sizeof(double) * 6 * (size_t)(pf + 1) * tb;
 }
 
-// the FP64 form's Helmholtz solves: one lane per column while the columns fill the SMs, one per
-// column, field and part below (k_helm64)
-static bool helm64_split(const lh_handle *h) { return h->g.nvc < LH_H64_SPLIT; }
+// the FP64 form's Helmholtz solves: fused (k_helm64), or right-hand sides and sweeps of their own
 static void launch_helm64_v(lh_handle *h, int kRK, cudaStream_t st) {
   Helm64Args a = {{(double *)h->u2, nullptr}, {(double *)h->Nu2, nullptr}, {(const double *)h->N2xz, nullptr},
                   {(const double *)h->vvc, nullptr}, (const double *)h->p, h->a3v, h->ib ? h->d_ibslot_v : nullptr,
                   (const double *)h->duib, kRK};
-  const int nl = h->g.nv, n = h->g.nvc;
-  if (helm64_split(h)) k_helm64<true, 1, 1><<<(2 * n + LH_H64_T - 1) / LH_H64_T, LH_H64_T, helm64_smem(true, 1, 1, nl), st>>>(a, h->g, h->sc);
-  else k_helm64<true, 1, 2><<<(n + LH_H64_T - 1) / LH_H64_T, LH_H64_T, helm64_smem(true, 1, 2, nl), st>>>(a, h->g, h->sc);
+  k_helm64<true><<<(h->g.nvc + LH_H64_T - 1) / LH_H64_T, LH_H64_T, helm64_smem(true, h->g.nv), st>>>(a, h->g, h->sc);
 }
 static void launch_helm64_uw(lh_handle *h, int kRK) {
   Helm64Args a = {{(double *)h->u1, (double *)h->u3}, {(double *)h->Nu1, (double *)h->Nu3},
                   {(const double *)h->N1xz, (const double *)h->N3xz}, {(const double *)h->uvf, (const double *)h->wvf},
                   (const double *)h->p, h->a3s, h->ib ? h->d_ibslot_u : nullptr, (const double *)h->duib, kRK};
-  const int nl = h->g.nu, n = h->g.nvc;
-  if (helm64_split(h)) {
-    const dim3 grid((2 * n + LH_H64_T - 1) / LH_H64_T, 2);
-    k_helm64<false, 1, 1><<<grid, LH_H64_T, helm64_smem(false, 1, 1, nl), h->st>>>(a, h->g, h->sc);
-  } else {
-    k_helm64<false, 2, 2><<<(n + LH_H64_T - 1) / LH_H64_T, LH_H64_T, helm64_smem(false, 2, 2, nl), h->st>>>(a, h->g, h->sc);
-  }
+  k_helm64<false><<<(h->g.nvc + LH_H64_T - 1) / LH_H64_T, LH_H64_T, helm64_smem(false, h->g.nu), h->st>>>(a, h->g, h->sc);
+}
+static bool helm_split(const lh_handle *h) { return h->prec == LH_PREC_FP64 && h->g.nvc < LH_HELM_SPLIT; }
+static int launch_helm_split(lh_handle *h, int kRK) {
+  const Geo &g = h->g;
+  const size_t n = 2 * (size_t)g.nu * g.ncol;
+  const int *iu = h->ib ? h->d_ibslot_u : nullptr, *iv = h->ib ? h->d_ibslot_v : nullptr;
+  HelmArgs a = {{h->u1, h->u3, h->u2},
+                {(double2 *)h->Nu1, (double2 *)h->Nu3, (double2 *)h->Nu2},
+                {(double2 *)h->N1xz, (double2 *)h->N3xz, (double2 *)h->N2xz},
+                {(const double2 *)h->uvf, (const double2 *)h->wvf, (const double2 *)h->vvc},
+                h->p, {h->a3s, h->a3s + n, h->a3v}, {iu, iu, iv}, (const double2 *)h->duib, kRK};
+  KL("k_helm_rhs", k_helm_rhs<<<dim3(3 * ((g.nvc + 127) / 128), (g.nu + LH_HL - 1) / LH_HL), 128, 0, h->st>>>(a, g, h->sc));
+  KL("k_helm_sweep", k_helm_sweep64<<<dim3((2 * g.nvc + LH_HS_T - 1) / LH_HS_T, 3), LH_HS_T, hsweep_smem(g.nu), h->st>>>(a, g, h->sc));
+  return LH_OK;
 }
 
 template <typename T>
@@ -1334,26 +1337,29 @@ static int substep_launches_t(lh_handle *h, int kRK) {
     CK(cudaEventRecord(h->ev_fork, h->st));
     CK(cudaStreamWaitEvent(h->st2, h->ev_fork, 0));
   }
-  if (!fork) prof_begin(h, "k_helm_v");
-  if (h->prec == LH_PREC_FP64) {
-    launch_helm64_v(h, kRK, sv);
-  } else {
-    const int nb2v = (2 * g.nvc + h->tb_v - 1) / h->tb_v;
-    const size_t sm = staged_smem(g.nv, h->pf_v, h->tb_v);
-    const int *ibv = h->ib ? h->d_ibslot_v : nullptr;
-    double *V = (double *)h->u2;
-    float *NV = (float *)h->Nu2;
-    const float *XV = (const float *)h->N2xz, *VV = (const float *)h->vvc;
-    const double *PP = (const double *)h->p;
-    float2 *YS = (float2 *)h->ysv;
-    switch (h->pf_v) {
-      case 0: k_helm_v_mx2<<<nb2v, h->tb_v, 0, sv>>>(V, NV, XV, VV, PP, YS, g, h->sc, kRK, ibv, (const float2 *)h->duib); break;
-      case 2: k_helm_v_mx3<2><<<nb2v, h->tb_v, sm, sv>>>(V, NV, XV, VV, PP, YS, g, h->sc, kRK, ibv, (const float2 *)h->duib); break;
-      case 8: k_helm_v_mx3<8><<<nb2v, h->tb_v, sm, sv>>>(V, NV, XV, VV, PP, YS, g, h->sc, kRK, ibv, (const float2 *)h->duib); break;
-      default: k_helm_v_mx3<4><<<nb2v, h->tb_v, sm, sv>>>(V, NV, XV, VV, PP, YS, g, h->sc, kRK, ibv, (const float2 *)h->duib); break;
+  const bool hsplit = helm_split(h);
+  if (!hsplit) {
+    if (!fork) prof_begin(h, "k_helm_v");
+    if (h->prec == LH_PREC_FP64) {
+      launch_helm64_v(h, kRK, sv);
+    } else {
+      const int nb2v = (2 * g.nvc + h->tb_v - 1) / h->tb_v;
+      const size_t sm = staged_smem(g.nv, h->pf_v, h->tb_v);
+      const int *ibv = h->ib ? h->d_ibslot_v : nullptr;
+      double *V = (double *)h->u2;
+      float *NV = (float *)h->Nu2;
+      const float *XV = (const float *)h->N2xz, *VV = (const float *)h->vvc;
+      const double *PP = (const double *)h->p;
+      float2 *YS = (float2 *)h->ysv;
+      switch (h->pf_v) {
+        case 0: k_helm_v_mx2<<<nb2v, h->tb_v, 0, sv>>>(V, NV, XV, VV, PP, YS, g, h->sc, kRK, ibv, (const float2 *)h->duib); break;
+        case 2: k_helm_v_mx3<2><<<nb2v, h->tb_v, sm, sv>>>(V, NV, XV, VV, PP, YS, g, h->sc, kRK, ibv, (const float2 *)h->duib); break;
+        case 8: k_helm_v_mx3<8><<<nb2v, h->tb_v, sm, sv>>>(V, NV, XV, VV, PP, YS, g, h->sc, kRK, ibv, (const float2 *)h->duib); break;
+        default: k_helm_v_mx3<4><<<nb2v, h->tb_v, sm, sv>>>(V, NV, XV, VV, PP, YS, g, h->sc, kRK, ibv, (const float2 *)h->duib); break;
+      }
     }
+    if ((rc = count_launch(h))) return rc;
   }
-  if ((rc = count_launch(h))) return rc;
   const bool mixed00 = h->prec == LH_PREC_MIXED;
   if (mixed00) {
     const size_t sm00 = 8 * sizeof(double) * (size_t)(std::max(g.nu, g.nv) + 1);
@@ -1368,7 +1374,9 @@ static int substep_launches_t(lh_handle *h, int kRK) {
     if ((rc = meanflow(h, kRK, sv))) return rc;
     CK(cudaEventRecord(h->ev_mf, h->st2));
   }
-  if (h->prec == LH_PREC_FP64) {
+  if (hsplit) {
+    if ((rc = launch_helm_split(h, kRK))) return rc;
+  } else if (h->prec == LH_PREC_FP64) {
     KL("k_helm_uw", launch_helm64_uw(h, kRK));
   } else {
     const int nb2u = (2 * g.nvc + h->tb_uw - 1) / h->tb_uw;
@@ -1408,7 +1416,7 @@ static int substep_launches_t(lh_handle *h, int kRK) {
     const dim3 ge((g.nvc + 127) / 128, (g.np + LH_PL - 1) / LH_PL);
     double2 *vlow = need_div ? (double2 *)h->A : nullptr;  // (the transforms' scratch is free here)
     KL("k_press_rhs", k_press_rhs<<<ge, 128, 0, h->st>>>(h->u1, h->u2, h->u3, h->psi, vlow, g, h->sc, kRK));
-    KL("k_press", k_press_sweep<<<(2 * g.nvc + 31) / 32, 32, 0, h->st>>>((double *)h->psi, h->dg1, h->dg2, h->dg3, g));
+    KL("k_press_sweep", k_press_sweep<<<(2 * g.nvc + 31) / 32, 32, 0, h->st>>>((double *)h->psi, h->dg1, h->dg2, h->dg3, g));
     if (mf_side) CK(cudaStreamWaitEvent(h->st, h->ev_mf, 0));
     if (need_div) KL("k_press_corr", k_press_corr<true><<<ge, 128, 0, h->st>>>(h->u1, h->u2, h->u3, h->p, h->psi, vlow, g, h->sc, kRK));
     else KL("k_press_corr", k_press_corr<false><<<ge, 128, 0, h->st>>>(h->u1, h->u2, h->u3, h->p, h->psi, vlow, g, h->sc, kRK));

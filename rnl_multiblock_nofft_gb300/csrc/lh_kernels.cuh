@@ -280,33 +280,20 @@ template <int N> __device__ __forceinline__ void cpa_wait() { asm volatile("cp.a
 // backward sweep writes the solution in place. At immersed-boundary levels du is read from
 // `duib` (assembled and forced beforehand) instead of being formed here.
 //
-// A lane carries NF fields (u and w share their matrix) and NP parts (real, imaginary) of one
-// column; field blockIdx.y + 0 .. NF-1, part (lane % (2 / NP)).
-//  - Large channels, <2, 2> and v <1, 2>: bound by the FP64 pipe (2 operations a clock and SM), so
-//    one lane does everything that shares the factorisation, and the operations are few: the
-//    row l of -dt / Re L serves the matrix (I + bRK l) and the right-hand side (-aRK l u), and
-//    dt is folded into the other coefficients. u/w 93 -> 66 and v 65 -> 42 operations a column level.
-//  - Small channels, <1, 1>: bound by the serial chain of a level (reciprocal and two fused
-//    operations, ~1/3 of a microsecond) and by the FP64 issue of the few SMs that hold the
-//    columns, so the components spread over four times as many lanes (each repeats the
-//    factorisation).
-// The level's inputs come D levels ahead through a cp.async ring in shared memory. 32-thread
-// blocks spread the columns evenly over the 152 SMs (1032 blocks at 256 x 256: 6.8 a SM).
-// Measured at 256 x 256 x 301 with posts / 32 x 32 x 153, ms per step, against one lane per
-// column with all operations in the reference's order: u/w 5.63 -> 4.32 / 1.32 -> 0.49, v 3.94 -> 2.89 / 0.89 -> 0.49
-// (both run together in the step: FP64 pipe 82-86 % busy).
+// A lane carries a column segment's fields (u and w share their matrix; v) and both parts. The
+// FP64 pipe (2 operations a clock and SM) bounds the kernel, so one lane does everything that
+// shares the factorisation, and the operations are few: the row l of -dt / Re L serves the matrix
+// (I + bRK l) and the right-hand side (-aRK l u), and dt is folded into the other coefficients.
+// u/w 93 -> 66 and v 65 -> 42 operations a column level. The level's inputs come D levels ahead
+// through a cp.async ring in shared memory. 32-thread blocks spread the columns evenly over the
+// 152 SMs (1032 blocks at 256 x 256: 6.8 a SM). Small channels: k_helm_rhs and k_helm_sweep64.
+// Measured at 256 x 256 x 301 with posts, ms per step, against one lane per column with all
+// operations in the reference's order: u/w 5.63 -> 4.32, v 3.94 -> 2.89 (both run together in the
+// step: FP64 pipe 82-86 % busy).
 // ============================================================================
 #define LH_H64_D 2   // levels ahead
 #define LH_H64_T 32  // threads per block
-// columns below which the components spread over lanes: twice the lanes that one warp per SM holds
-#define LH_H64_SPLIT 2432
-template <int NP> struct Part;
-template <> struct Part<2> { typedef double2 t; };
-template <> struct Part<1> { typedef double t; };
 __device__ __forceinline__ double &comp(double2 &v, int s) { return s ? v.y : v.x; }
-__device__ __forceinline__ double &comp(double &v, int) { return v; }
-__device__ __forceinline__ void cpa_part(double2 *d, const double *s) { cpa16(d, s); }
-__device__ __forceinline__ void cpa_part(double *d, const double *s) { cpa8(d, s); }
 
 struct Helm64Args {
   double *u[2];          // the fields (v: [0])
@@ -314,23 +301,23 @@ struct Helm64Args {
   const double *X[2];    // N_xz
   const double *F[2];    // y-flux
   const double *p;
-  double *a3s;           // upper factors [field group][level][column]
+  double *a3s;           // upper factors [level][column]
   const int *ibslot;
   const double *duib;
   int kRK;
 };
-__host__ __device__ constexpr int helm64_entries(bool V, int NF) { return V ? 5 : 1 + 4 * NF; }
+__host__ __device__ constexpr int helm64_entries(bool V) { return V ? 5 : 9; }
 // bytes: the level tables (row of -dt / Re L without k^2, d/dy factor, immersed slot) and the ring
-__host__ __device__ constexpr size_t helm64_smem(bool V, int NF, int NP, int nlev) {
-  return (((size_t)nlev * 36 + 15) & ~(size_t)15) +
-         (size_t)helm64_entries(V, NF) * (LH_H64_D + 1) * LH_H64_T * 8 * NP;
+__host__ __device__ constexpr size_t helm64_smem(bool V, int nlev) {
+  return (((size_t)nlev * 36 + 15) & ~(size_t)15) + (size_t)helm64_entries(V) * (LH_H64_D + 1) * LH_H64_T * 16;
 }
 
 // V: the wall-normal velocity (levels at the faces; gradient and flux differences across them)
-template <bool V, int NF, int NP>
+template <bool V>
 __global__ void __launch_bounds__(LH_H64_T) k_helm64(Helm64Args a, Geo g, const DevScalars *__restrict__ sc) {
-  typedef typename Part<NP>::t T;
-  constexpr int D = LH_H64_D, NS = D + 1, NT = LH_H64_T, NE = helm64_entries(V, NF);
+  typedef double2 T;
+  constexpr int NF = V ? 1 : 2, NP = 2;  // fields, parts
+  constexpr int D = LH_H64_D, NS = D + 1, NT = LH_H64_T, NE = helm64_entries(V);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int nlev = V ? g.nv : g.nu, kRK = a.kRK;
   double *t1 = reinterpret_cast<double *>(smem_raw), *t2 = t1 + nlev, *t3 = t2 + nlev, *tth = t3 + nlev;
@@ -347,48 +334,45 @@ __global__ void __launch_bounds__(LH_H64_T) k_helm64(Helm64Args a, Geo g, const 
     }
   }
   __syncthreads();
-  const int lane = blockIdx.x * NT + threadIdx.x;
-  const int vc = NP == 2 ? lane : lane >> 1, part = NP == 2 ? 0 : lane & 1;
+  const int vc = blockIdx.x * NT + threadIdx.x;
   const int nc = g.ncol;
   if (vc >= g.nvc) return;
   int c, bd;
   vcol_of(g, vc, c, bd);
   const int qlo = g.bq[bd][V ? 2 : 0], qhi = g.bq[bd][V ? 3 : 1];
   const int r = c / g.N1h, kx = c - r * g.N1h;
-  const int fy = NF == 2 || V ? 0 : (int)blockIdx.y;
   const double uk = unit * (g.k2x[kx] + g.k2z[r]);
   const double aR = g.aRK[kRK - 1], bR = g.bRK[kRK - 1];
   const double c2 = -dt * g.cRK[kRK - 1], cg = -dt * g.gRK[kRK - 1], cp = -dt * g.dRK[kRK - 1];
   const double mp = (!V && c == 0) ? cp * sc->mpgx : 0.0;  // u only, real part
   const double gw0 = V ? 0.0 : g.gw[bd][0], gw1 = V ? 0.0 : g.gw[bd][1];
-  const size_t ls = (size_t)nc * 2, ci = (size_t)c * 2 + part, co = (size_t)c * 2 + (NP == 1 ? part ^ 1 : 0);
+  const size_t ls = (size_t)nc * 2, ci = (size_t)c * 2;
   double *u[NF], *No[NF];
   const double *X[NF], *F[NF];
   double ck[NF];  // -dt dRK k of the field's gradient
   int fd[NF];     // field in duib
 #pragma unroll
   for (int f = 0; f < NF; ++f) {
-    const bool w = f == 1 || fy == 1;
-    u[f] = (w ? a.u[1] : a.u[0]) + ci; No[f] = (w ? a.Nu[1] : a.Nu[0]) + ci;
-    X[f] = (w ? a.X[1] : a.X[0]) + ci; F[f] = (w ? a.F[1] : a.F[0]) + ci;
-    ck[f] = V ? 0.0 : cp * (f + fy ? g.k1z[r] : g.k1x[kx]);
-    fd[f] = V ? 1 : (f + fy ? 2 : 0);
+    u[f] = a.u[f] + ci; No[f] = a.Nu[f] + ci;
+    X[f] = a.X[f] + ci; F[f] = a.F[f] + ci;
+    ck[f] = V ? 0.0 : cp * (f ? g.k1z[r] : g.k1x[kx]);
+    fd[f] = V ? 1 : 2 * f;
   }
-  double *a3 = a.a3s + (size_t)fy * (NP == 1 ? 2 : 1) * nlev * nc + (size_t)part * nlev * nc + c;
+  double *a3 = a.a3s + c;
 #define RS(s_, k_) ring[((s_) * NE + (k_)) * NT + threadIdx.x]
   // slot of level q: the fields one level up, p, Nu, X, flux (v: v one level up, p at q, Nu, X, vv one up)
   auto fetch = [&](int q) {
     const int s_ = (q - qlo - 1) % NS;
     const size_t o = (size_t)q * ls;
     if (V) {
-      cpa_part(&RS(s_, 0), u[0] + o + ls); cpa_part(&RS(s_, 1), a.p + o + ci);
-      cpa_part(&RS(s_, 2), No[0] + o); cpa_part(&RS(s_, 3), X[0] + o); cpa_part(&RS(s_, 4), F[0] + o + ls);
+      cpa16(&RS(s_, 0), u[0] + o + ls); cpa16(&RS(s_, 1), a.p + o + ci);
+      cpa16(&RS(s_, 2), No[0] + o); cpa16(&RS(s_, 3), X[0] + o); cpa16(&RS(s_, 4), F[0] + o + ls);
     } else {
-      cpa_part(&RS(s_, 0), a.p + o - ls + co);
+      cpa16(&RS(s_, 0), a.p + o - ls + ci);
 #pragma unroll
       for (int f = 0; f < NF; ++f) {
-        cpa_part(&RS(s_, 1 + 4 * f), u[f] + o + ls); cpa_part(&RS(s_, 2 + 4 * f), No[f] + o);
-        cpa_part(&RS(s_, 3 + 4 * f), X[f] + o); cpa_part(&RS(s_, 4 + 4 * f), F[f] + o);
+        cpa16(&RS(s_, 1 + 4 * f), u[f] + o + ls); cpa16(&RS(s_, 2 + 4 * f), No[f] + o);
+        cpa16(&RS(s_, 3 + 4 * f), X[f] + o); cpa16(&RS(s_, 4 + 4 * f), F[f] + o);
       }
     }
   };
@@ -444,10 +428,8 @@ __global__ void __launch_bounds__(LH_H64_T) k_helm64(Helm64Args a, Geo g, const 
           if (V) {
             v += (cp * th) * (comp(w[1], s) - comp(pm, s));
           } else {  // i k p: the other part, with its sign
-            const double pk = NP == 2 ? comp(w[0], s ^ 1) : comp(w[0], 0);
-            const bool re = NP == 2 ? s == 0 : part == 0;
-            v += (re ? -ck[f] : ck[f]) * pk;
-            if (f + fy == 0 && re) v += mp;
+            v += (s ? ck[f] : -ck[f]) * comp(w[0], s ^ 1);
+            if (f == 0 && s == 0) v += mp;
           }
           comp(rhs, s) = comp(u0[f], s) + v;
         }
@@ -482,7 +464,7 @@ __global__ void __launch_bounds__(LH_H64_T) k_helm64(Helm64Args a, Geo g, const 
   auto fetch_b = [&](int q) {
     const int s_ = (qhi - 1 - q) % NS;
 #pragma unroll
-    for (int f = 0; f < NF; ++f) cpa_part(&ring[(s_ * NF + f) * NT + threadIdx.x], u[f] + (size_t)q * ls);
+    for (int f = 0; f < NF; ++f) cpa16(&ring[(s_ * NF + f) * NT + threadIdx.x], u[f] + (size_t)q * ls);
     cpa8(&ra[s_ * NT + threadIdx.x], a3 + (size_t)q * nc);
   };
 #pragma unroll
@@ -1200,6 +1182,212 @@ __global__ void __launch_bounds__(NTHR) k_helm_v_mx3(double *__restrict__ u2, fl
   }
   __threadfence_block();
   back_sweep_staged<D>(u2, ys, lstride, ci, qlo, qhi, y, ring, nt);
+}
+
+// ============================================================================
+// Helmholtz solves of the FP64 form below LH_HELM_SPLIT columns (two lanes a column and field: two
+// warps a scheduler): the right-hand sides element-wise over (column, chunk of levels), then the
+// sweeps alone. An FP64 warp instruction holds its scheduler's half lane a clock for 64 cycles;
+// a fused sweep with a lane per component held 26 of them a level, alone it holds the
+// factorisation and three. (In the mixed form the same split was faster for a channel alone and
+// 6 % slower for an ensemble, whose channels fill the GPU together.) The right-hand side takes
+// the place of N_xz, which nothing reads after it, and the sweep's y that of the right-hand side.
+// 32 x 32 x 153, us a launch of the fused sweep u/w 165, v 164 (side by side) -> 23 + 76.
+// ============================================================================
+#define LH_HL 8  // levels of a thread of the right-hand sides
+#define LH_HELM_SPLIT 2432
+struct HelmArgs {
+  double2 *u[3];           // u, w, v
+  double2 *Nu[3], *X[3];   // previous nonlinear terms; N_xz, then the right-hand side, then y
+  const double2 *F[3];     // y-flux: uv, wv, vv
+  const double2 *p;
+  double *a3[3];           // upper factors [level][column][part]
+  const int *ibslot[3];
+  const double2 *duib;     // [slot][field u, v, w][column]
+  int kRK;
+};
+
+// Right-hand side u + dt du of one field at the interior levels q0 .. q1 - 1 of a column segment
+// (both parts), as k_helm64 forms it; V: v
+template <bool V>
+__device__ __forceinline__ void helm_rhs_field(const HelmArgs &a, const Geo &g, const DevScalars *__restrict__ sc, int f,
+                                               int c, int q0, int q1) {
+  const int kRK = a.kRK, nc = g.ncol, r = c / g.N1h, kx = c - r * g.N1h, nl = V ? g.nv : g.nu;
+  double2 *u = a.u[f];
+  double2 *Nu = a.Nu[f], *X = a.X[f];
+  const double2 *F = a.F[f];
+  const int *ibslot = a.ibslot[f];
+  const int fd = V ? 1 : 2 * f;
+  const double dt = sc->dt, dR = g.dRK[kRK - 1];
+  size_t e = (size_t)q0 * nc + c;
+  double2 um = u[e - nc], u0 = u[e];
+  double2 fl = V ? F[e] : F[e - nc];
+  double2 pm;
+  if (V) pm = a.p[e - nc];
+      const double unit = -dt / g.Re * g.aRK[kRK - 1], k2 = g.k2x[kx] + g.k2z[r];
+      const double c2 = -dt * g.cRK[kRK - 1], cg = -dt * g.gRK[kRK - 1], cp = -dt * dR;
+      const double ck = V ? 0.0 : cp * (f ? g.k1z[r] : g.k1x[kx]);
+      const double mp = (f == 0 && c == 0) ? cp * sc->mpgx : 0.0;  // u only, real part
+      const double *d2 = V ? g.d2v : g.d2u, *th = V ? g.thv : g.thu;
+  #pragma unroll 2
+      for (int q = q0; q < q1; ++q, e += nc) {
+        const double2 up1 = u[e + nc], pq = a.p[V ? e : e - nc];
+        const double2 fq = V ? F[e + nc] : F[e], nuq = Nu[e], xq = X[e];
+        const double l1 = unit * d2[q], l2 = unit * (d2[nl + q] + k2), l3 = unit * d2[2 * nl + q], thq = th[q] * g.dd;
+        const int ibs = ibslot ? ibslot[q] : -1;
+        double2 rr, nn;
+  #pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          const double upt = t ? up1.y : up1.x, u0t = t ? u0.y : u0.x, umt = t ? um.y : um.x;
+          const double flq = t ? fq.y : fq.x, flm = t ? fl.y : fl.x, nu = t ? nuq.y : nuq.x, x = t ? xq.y : xq.x;
+          double v;
+          if (ibs < 0) {
+            const double n = x + (flq - flm) * thq;
+            (t ? nn.y : nn.x) = n;
+            v = c2 * nu - (l1 * umt + (l2 * u0t + l3 * upt));  // the increment first: u's rounding enters once
+            v += cg * n;
+            if (V) {
+              v += (cp * thq) * (t ? pq.y - pm.y : pq.x - pm.x);
+            } else {
+              v += t ? ck * pq.x : -ck * pq.y;
+              if (t == 0) v += mp;
+            }
+          } else {
+            const double2 di = a.duib[((size_t)ibs * 3 + fd) * nc + c];
+            v = dt * (t ? di.y : di.x);
+          }
+          (t ? rr.y : rr.x) = u0t + v;
+        }
+        if (ibs < 0) { Nu[e].x = nn.x; Nu[e].y = nn.y; }
+        X[e].x = rr.x; X[e].y = rr.y;
+        um = u0; u0 = up1; fl = fq;
+        if (V) pm = pq;
+      }
+}
+// grid: x = (column block, field), y = chunk of levels
+__global__ void __launch_bounds__(128) k_helm_rhs(HelmArgs a, Geo g, const DevScalars *__restrict__ sc) {
+  const int f = blockIdx.x % 3, vc = (blockIdx.x / 3) * 128 + threadIdx.x;
+  if (vc >= g.nvc) return;
+  int c, bd;
+  vcol_of(g, vc, c, bd);
+  const int qlo = g.bq[bd][f == 2 ? 2 : 0], qhi = g.bq[bd][f == 2 ? 3 : 1];
+  const int q0 = qlo + 1 + blockIdx.y * LH_HL, q1 = min(q0 + LH_HL, qhi);
+  if (q0 >= q1) return;
+  if (f == 2) helm_rhs_field<true>(a, g, sc, 2, c, q0, q1);
+  else helm_rhs_field<false>(a, g, sc, f, c, q0, q1);
+}
+
+// The sweeps of one field: lane = (column segment, part), field blockIdx.y. U levels a batch, two
+// batches ahead. The level tables are the matrix rows without k^2.
+#define LH_HS_U 4
+#define LH_HS_T 64
+__host__ __device__ constexpr int hsweep_region() { return (3 * LH_HS_U * 2) | 1; }  // doubles of a thread's ring
+__host__ __device__ constexpr size_t hsweep_smem(int nlev) { return 8 * ((size_t)3 * nlev + LH_HS_T * hsweep_region()); }
+__global__ void __launch_bounds__(LH_HS_T) k_helm_sweep64(HelmArgs a, Geo g, const DevScalars *__restrict__ sc) {
+  constexpr int U = LH_HS_U, EL = 2, BE = U * EL;  // a level: y, factor (backward)
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int f = blockIdx.y, kRK = a.kRK, nlev = f == 2 ? g.nv : g.nu;
+  double *ring_all = reinterpret_cast<double *>(smem_raw), *ta = ring_all + LH_HS_T * hsweep_region(), *tb = ta + nlev,
+         *tc = tb + nlev;
+  const double beta = g.bRK[kRK - 1] * sc->dt / g.Re;
+  {
+    const double *d2 = f == 2 ? g.d2v : g.d2u;
+    for (int i = threadIdx.x; i < nlev; i += LH_HS_T) {
+      ta[i] = -beta * d2[i]; tb[i] = 1.0 - beta * d2[nlev + i]; tc[i] = -beta * d2[2 * nlev + i];
+    }
+  }
+  __syncthreads();
+  double *ring = ring_all + threadIdx.x * hsweep_region();
+  const unsigned rs = (unsigned)__cvta_generic_to_shared(ring);
+  const int tid = blockIdx.x * LH_HS_T + threadIdx.x, vc = tid >> 1, part = tid & 1;
+  if (vc >= g.nvc) return;
+  int c, bd;
+  vcol_of(g, vc, c, bd);
+  const bool V = f == 2;
+  const int qlo = g.bq[bd][V ? 2 : 0], qhi = g.bq[bd][V ? 3 : 1];
+  const size_t ls = 2 * (size_t)g.ncol, ci = 2 * (size_t)c + part;
+  const int r = c / g.N1h, kx = c - r * g.N1h;
+  const double bk = beta * (g.k2x[kx] + g.k2z[r]);
+  const double gw1 = V ? 0.0 : g.gw[bd][0], gw2 = V ? 0.0 : g.gw[bd][1];
+  double *u = reinterpret_cast<double *>(a.u[f]) + ci, *X = reinterpret_cast<double *>(a.X[f]) + ci, *A = a.a3[f] + ci;
+  double y = 0.0, a3raw = gw1, a2p = 1.0;  // first row: [1, gw(b,1)], rhs 0
+  {
+    const double *fx = X + (size_t)(qlo + 1) * ls;
+    int left = qhi - qlo - 1;
+    unsigned dst = rs;
+    auto fetch = [&]() {
+#pragma unroll
+      for (int i = 0; i < U; ++i)
+        if (left > i) { cpa8s(dst + 8 * i, fx); fx += ls; }
+      left -= U;
+      dst = dst == rs + 8 * 2 * BE ? rs : dst + 8 * BE;
+      cpa_commit();
+    };
+    fetch();
+    fetch();
+    double *oy = X + (size_t)(qlo + 1) * ls, *oa = A + (size_t)qlo * ls;
+    const double *h = ring;
+    int q = qlo + 1;
+    for (int n = qhi - qlo - 1; n > 0; n -= U) {
+      fetch();
+      cpa_wait<2>();
+#pragma unroll
+      for (int i = 0; i < U; ++i) {
+        if (i > 0 && n <= i) break;
+        const double rr = h[i], a1 = ta[q + i], a2 = tb[q + i] - bk;
+        const double a3p = a3raw * a2p;
+        *oa = a3p;
+        oa += ls;
+        a2p = 1.0 / (a2 - a1 * a3p);
+        y = (rr - a1 * y) * a2p;
+        *oy = y;
+        oy += ls;
+        a3raw = tc[q + i];
+      }
+      q += U;
+      h = h == ring + 2 * BE ? ring : h + BE;
+    }
+  }
+  cpa_wait<0>();
+  {  // last row: [gw(b,2), 1], rhs 0
+    const double a3p = a3raw * a2p;
+    A[(size_t)(qhi - 1) * ls] = a3p;
+    a2p = 1.0 / (1.0 - gw2 * a3p);
+    y = (0.0 - gw2 * y) * a2p;
+    u[(size_t)qhi * ls] = y;
+  }
+  __threadfence();  // the copies below read what this thread stored above
+  {
+    const double *fy = X + (size_t)(qhi - 1) * ls, *fa = A + (size_t)(qhi - 1) * ls;
+    double *ou = u + (size_t)(qhi - 1) * ls;
+    int left = qhi - qlo;
+    unsigned dst = rs;
+    auto fetch = [&]() {
+#pragma unroll
+      for (int i = 0; i < U; ++i)
+        if (left > i) { cpa8s(dst + 16 * i, fy); cpa8s(dst + 16 * i + 8, fa); fy -= ls; fa -= ls; }
+      left -= U;
+      dst = dst == rs + 8 * 2 * BE ? rs : dst + 8 * BE;
+      cpa_commit();
+    };
+    fetch();
+    fetch();
+    const double *h = ring;
+    for (int n = qhi - qlo; n > 0; n -= U) {
+      fetch();
+      cpa_wait<2>();
+#pragma unroll
+      for (int i = 0; i < U; ++i) {
+        if (i > 0 && n <= i) break;
+        const double ya = n == i + 1 ? 0.0 : h[2 * i], a3p = h[2 * i + 1];
+        y = ya - a3p * y;
+        *ou = y;
+        ou -= ls;
+      }
+      h = h == ring + 2 * BE ? ring : h + BE;
+    }
+  }
+  cpa_wait<0>();
 }
 
 // ============================================================================
