@@ -88,6 +88,7 @@ struct lh_handle {
   int tri_threads;
   size_t tri_smem;
   long long tri_nterms;
+  long long beside;  // columns of the other channels of the batch being captured
   cudaGraph_t graph;
   cudaGraphExec_t gexec;
   bool graph_ready;
@@ -1331,7 +1332,8 @@ static int substep_launches_t(lh_handle *h, int kRK) {
   // the mean-flow correction, which changes u(0,0) alone, follows it there. (Sequential on the
   // main stream while per-kernel times are profiled.)
   const bool fork = !h->prof;
-  const bool split = g.nvc < LH_PRESS_SPLIT_COLS;
+  // (fused and split pressure steps have the same results bit for bit)
+  const bool split = g.nvc + h->beside < LH_PRESS_SPLIT_COLS;
   cudaStream_t sv = fork ? h->st2 : h->st;
   if (fork) {
     CK(cudaEventRecord(h->ev_fork, h->st));
@@ -1925,11 +1927,15 @@ extern "C" int lh_batch_create(lh_handle *const *handles, int n, lh_batch **out)
   cudaEventRecord(b->ev0, b->root);
   int rc = LH_OK;
   std::string why;
+  long long cols = 0;
+  for (lh_handle *h : b->hs) cols += h->g.nvc;
   for (int i = 0; i < n && rc == LH_OK; ++i) {
     lh_handle *h = b->hs[i];
     cudaStreamWaitEvent(h->st, b->ev0, 0);
     long long before = h->launches;
+    h->beside = cols - h->g.nvc;
     rc = step_launches(h);
+    h->beside = 0;
     h->launches = before;
     if (rc != LH_OK) why = "channel " + std::to_string(i) + ": " + h->err;
     cudaEventRecord(b->evs[i], h->st);

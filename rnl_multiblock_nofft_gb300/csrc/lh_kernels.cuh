@@ -1931,6 +1931,9 @@ __global__ void __launch_bounds__(NTHR) k_press3(double *__restrict__ u1, double
 // columns) 143 -> 59, 128 x 96 x 201 (6240) 190 -> 127. us a step, mixed form alone / among others:
 // 128 x 128 x 201 (8320) 1784 / 1330 -> 1555 / 1263, 192 x 128 x 201 (12416) 2368 / 2004 -> 2184 /
 // 2003, 192 x 192 x 201 (18624) 3025 / 2936 -> 3100 / 3038.
+// In a batch the columns of all its channels count: they run beside each other, so the split route's
+// extra launches and traffic cost what they cost a large channel (16 uneven channels: 4233 us a step
+// split, 4214 fused; 4211 before there was a choice).
 // ============================================================================
 #define LH_PRESS_SPLIT_COLS 16384
 #define LH_PL 8  // levels of a thread of the element-wise kernels (rolling v, psi)
