@@ -2416,9 +2416,10 @@ __global__ void k_band_io(double2 *__restrict__ dev, double2 *__restrict__ stage
   else stage[i] = *d;
 }
 
-// host cfield [col][lev] <-> device [lev][col] (complex), tiled transpose
-__global__ void k_transpose(const double2 *__restrict__ src, double2 *__restrict__ dst, int rows, int cols) {
-  __shared__ double2 tile[32][33];
+// host cfield [col][lev] <-> device [lev][col] (complex; real for the spectra), tiled transpose
+template <typename V>
+__global__ void k_transpose(const V *__restrict__ src, V *__restrict__ dst, int rows, int cols) {
+  __shared__ V tile[32][33];
   const int bx = blockIdx.x * 32, by = blockIdx.y * 32;
   for (int i = threadIdx.y; i < 32; i += blockDim.y) {
     const int rr = by + i, cc = bx + threadIdx.x;
