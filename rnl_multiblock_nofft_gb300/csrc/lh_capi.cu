@@ -1106,7 +1106,7 @@ static int launch_zfwd(lh_handle *h, const Geo &g, int nslots, const void *twz) 
   } else {  // FP64: fixed point
     constexpr int KB = fx_kbf(N);
     dim3 grid((g.N1h + KB - 1) / KB, nslots);
-    KL("k_zfwd_nl", k_zfwd_fx<N><<<grid, fx_zt(N), fx_smem(N, 4 * KB), h->st>>>(
+    KL("k_zfwd_nl", k_zfwd_fx<N><<<grid, fx_ft(N), fx_smem(N, 4 * KB), h->st>>>(
                         (const double2 *)h->B, g, (const int4 *)twz, (double2 *)h->N1xz, (double2 *)h->N2xz,
                         (double2 *)h->N3xz, (double2 *)h->uvf, (double2 *)h->vvc, (double2 *)h->wvf));
   }
@@ -1180,14 +1180,14 @@ template <int N>
 static int launch_xinv_phys(lh_handle *h, const void *Ascr, double *phys, int npl, const void *twx) {
   constexpr int PB = fx_pbl(N);
   dim3 g2((h->g.G2 / 2 + PB - 1) / PB, npl);
-  KL("k_xinv_phys", k_xinv_phys_fx<N><<<g2, fx_xt(N), fx_smem(N, PB), h->st>>>((const double2 *)Ascr, phys, h->g, (const int4 *)twx));
+  KL("k_xinv_phys", k_xinv_phys_fx<N><<<g2, fx_lt(N), fx_smem(N, PB), h->st>>>((const double2 *)Ascr, phys, h->g, (const int4 *)twx));
   return LH_OK;
 }
 template <int N>
 static int launch_xfwd_phys(lh_handle *h, const double *phys, void *Bscr, int npl, const void *twx) {
   constexpr int PB = fx_pbl(N);
   dim3 g1((h->g.G2 / 2 + PB - 1) / PB, npl);
-  KL("k_xfwd_phys", k_xfwd_phys_fx<N><<<g1, fx_xt(N), fx_smem(N, PB), h->st>>>(phys, (double2 *)Bscr, h->g, (const int4 *)twx));
+  KL("k_xfwd_phys", k_xfwd_phys_fx<N><<<g1, fx_lt(N), fx_smem(N, PB), h->st>>>(phys, (double2 *)Bscr, h->g, (const int4 *)twx));
   return LH_OK;
 }
 template <typename T, int N>
@@ -1215,7 +1215,7 @@ static int launch_ib_xforce(lh_handle *h, int npl) {
   } else {  // FP64: fixed point
     constexpr int PB = fx_pbl(N);
     dim3 g2((h->g.G2 / 2 + PB - 1) / PB, npl);
-    KL("k_ib_xforce", k_ib_xforce_fx<N><<<g2, fx_xt(N), fx_smem(N, PB), h->st>>>(
+    KL("k_ib_xforce", k_ib_xforce_fx<N><<<g2, fx_lt(N), fx_smem(N, PB), h->st>>>(
                           (const double2 *)h->A, (double2 *)h->B, h->g, (const int4 *)h->twx, h->d_ibrec, h->d_iboff, (const double *)h->cap, h->sc));
   }
   return LH_OK;

@@ -16,19 +16,29 @@
 
 // threads and lines per block (the same values on the host). Lines are powers of two, so that
 // a thread of an interleaved pass works on one line and a warp holds every line equally often.
-#ifndef LH_FX_ZT
-#define LH_FX_ZT 192
-#endif
-#ifndef LH_FX_XT
-#define LH_FX_XT 192
-#endif
 __host__ __device__ constexpr int fx_pow2(int v) { return v >= 16 ? 16 : v >= 8 ? 8 : v >= 4 ? 4 : v >= 2 ? 2 : 1; }
 __host__ __device__ constexpr int fx_kbz(int n) { return fx_pow2(49152 / (32 * n)); }   // inverse z: columns
 __host__ __device__ constexpr int fx_kbf(int n) { return lh_clamp(fx_pow2(49152 / (128 * n)), 1, 8); }  // forward z: columns of four products
 __host__ __device__ constexpr int fx_pbx(int n) { return lh_clamp(fx_pow2(49152 / (128 * n)), 1, 8); }  // x: row pairs
-__host__ __device__ constexpr int fx_zt(int n) { return n > 384 ? 384 : LH_FX_ZT; }
-__host__ __device__ constexpr int fx_xt(int n) { return n > 384 ? 384 : LH_FX_XT; }
+__host__ __device__ constexpr int fx_pbl(int n) { return lh_clamp(fx_pow2(49152 / (32 * n)), 1, 16); }  // leaf x: row pairs, one line each
 __host__ __device__ constexpr size_t fx_smem(int n, int lines) { return (size_t)32 * n * lines; }  // two buffers
+// Threads of a block: as many as the stage with the most butterflies has, so that each stage is
+// one round (a stage of 256 butterflies on 192 threads is two, the second one third full), within
+// the registers of four blocks. ms a step against 192 (384 above a length of 384) everywhere,
+// inverse z / forward z: 384 (256 threads) .822 / 1.072 -> .778 / .939, 192 (256) .400 / .425 ->
+// .380 / .392, 144 (128) .264 / .272 -> .247 / .255, 576 (192, 320) 1.747 / 1.79 -> 1.346 / 1.81.
+// The x pass keeps 192 up to a length of 384: its instruction issue gains nothing from more warps
+// (384: 192 threads 2.401, 256 2.453; 192: .911, .953), and fewer suit 144 (192 .643, 128 .566).
+__host__ __device__ constexpr int fx_threads(int n, int lines, int most = 384) {
+  const int f = fx_first(n), s = fx_second(n), l = n / (f * s);
+  const int r = l > 1 && l < (f < s ? f : s) ? l : (f < s ? f : s);
+  const int blocks = 233472 / (32 * n * lines), cap = lh_clamp(1024 / lh_clamp(blocks, 1, 4) / 64 * 64, 128, most);
+  return lh_clamp((lines * (n / r) + 31) / 32 * 32, 128, cap);
+}
+__host__ __device__ constexpr int fx_zt(int n) { return fx_threads(n, fx_kbz(n)); }      // inverse z, leaf z
+__host__ __device__ constexpr int fx_ft(int n) { return fx_threads(n, 4 * fx_kbf(n)); }  // forward z
+__host__ __device__ constexpr int fx_xt(int n) { return fx_threads(n, 4 * fx_pbx(n), n > 384 ? 384 : 192); }  // x
+__host__ __device__ constexpr int fx_lt(int n) { return fx_threads(n, fx_pbl(n)); }      // leaf x
 
 // ---- scales of the lines of an interleaved pass -----------------------------------------
 // After each thread has put its elements of line (tid % KB) through hi / l1: the line's scale.
@@ -164,7 +174,7 @@ __device__ __forceinline__ const fx2 *fx_zfwd_stages(unsigned char *smem, const 
 template <int N, int NP, int KB>
 __device__ __forceinline__ void fx_zfwd_body(const double2 *__restrict__ B, const Geo &g, const int4 *__restrict__ tw,
                                              int q, int pbase, int kx0, double2 *oa, double2 *ob, double2 *oc) {
-  constexpr int NL = NP * KB, NT = fx_zt(N), NW = NT / 32;
+  constexpr int NL = NP * KB, NT = fx_ft(N), NW = NT / 32;
   static_assert(NT % NL == 0 && 32 % (2 * KB) == 0, "a thread keeps one column in each product and one line");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint2 slot[NW * NL];
@@ -237,7 +247,7 @@ __device__ __forceinline__ void fx_zfwd_body(const double2 *__restrict__ B, cons
 // level has two products instead of four and takes twice the columns, so that every block
 // carries the same lines.
 template <int N>
-__global__ void __launch_bounds__(fx_zt(N)) k_zfwd_fx(const double2 *__restrict__ B, Geo g, const int4 *__restrict__ tw,
+__global__ void __launch_bounds__(fx_ft(N)) k_zfwd_fx(const double2 *__restrict__ B, Geo g, const int4 *__restrict__ tw,
                                                       double2 *__restrict__ N1xz, double2 *__restrict__ N2xz,
                                                       double2 *__restrict__ N3xz, double2 *__restrict__ uvf,
                                                       double2 *__restrict__ vvc, double2 *__restrict__ wvf) {
@@ -578,10 +588,8 @@ __global__ void __launch_bounds__(fx_xt(N)) k_xpass_fx(const double2 *__restrict
 // Leaf plane transforms (k_xinv_phys, k_xfwd_phys), the immersed-boundary round trip
 // (k_ib_xforce) and the statistics' plane sums (k_xstats) on the same lines.
 // ============================================================================
-__host__ __device__ constexpr int fx_pbl(int n) { return lh_clamp(fx_pow2(49152 / (32 * n)), 1, 16); }  // row pairs, one line each
-
 template <int N>
-__global__ void __launch_bounds__(fx_xt(N)) k_xinv_phys_fx(const double2 *__restrict__ A, double *__restrict__ phys, Geo g,
+__global__ void __launch_bounds__(fx_lt(N)) k_xinv_phys_fx(const double2 *__restrict__ A, double *__restrict__ phys, Geo g,
                                                            const int4 *__restrict__ tw) {
   constexpr int PB = fx_pbl(N), NK = N / 3 + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -617,7 +625,7 @@ __device__ __forceinline__ void fx_rows_out(const fx2 *L, const FxScale *sc, dou
 }
 
 template <int N>
-__global__ void __launch_bounds__(fx_xt(N)) k_xfwd_phys_fx(const double *__restrict__ phys, double2 *__restrict__ B, Geo g,
+__global__ void __launch_bounds__(fx_lt(N)) k_xfwd_phys_fx(const double *__restrict__ phys, double2 *__restrict__ B, Geo g,
                                                            const int4 *__restrict__ tw) {
   constexpr int PB = fx_pbl(N), NK = N / 3 + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -637,7 +645,7 @@ __global__ void __launch_bounds__(fx_xt(N)) k_xfwd_phys_fx(const double *__restr
 }
 
 template <int N>
-__global__ void __launch_bounds__(fx_xt(N)) k_ib_xforce_fx(const double2 *__restrict__ A, double2 *__restrict__ B, Geo g,
+__global__ void __launch_bounds__(fx_lt(N)) k_ib_xforce_fx(const double2 *__restrict__ A, double2 *__restrict__ B, Geo g,
                                                            const int4 *__restrict__ tw, const IbRec *__restrict__ rec,
                                                            const int *__restrict__ rec_off, const double *__restrict__ cap,
                                                            const DevScalars *__restrict__ dsc) {
