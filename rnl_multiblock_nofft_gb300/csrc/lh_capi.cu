@@ -623,6 +623,7 @@ extern "C" int lh_create(const lh_config *cfg, lh_handle **out) {
         cudaFuncSetAttribute((const void *)k_press3<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
         cudaFuncSetAttribute((const void *)k_press3<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
         cudaFuncSetAttribute((const void *)k_helm_sweep64, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
+        cudaFuncSetAttribute((const void *)k_helm_sweep_mx, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
         cudaFuncSetAttribute((const void *)k_helm64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
         cudaFuncSetAttribute((const void *)k_helm64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
         cudaFuncSetAttribute((const void *)k_helm_u_mx3<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess ||
@@ -1278,8 +1279,26 @@ static void launch_helm64_uw(lh_handle *h, int kRK) {
                   (const double *)h->p, h->a3s, h->ib ? h->d_ibslot_u : nullptr, (const double *)h->duib, kRK};
   k_helm64<false><<<(h->g.nvc + LH_H64_T - 1) / LH_H64_T, LH_H64_T, helm64_smem(false, h->g.nu), h->st>>>(a, h->g, h->sc);
 }
-static bool helm_split(const lh_handle *h) { return h->prec == LH_PREC_FP64 && h->g.nvc < LH_HELM_SPLIT; }
+// (the mixed form's two routes have the same results bit for bit, so a batch may choose between them)
+static bool helm_split(const lh_handle *h) {
+  return h->prec == LH_PREC_FP64 ? h->g.nvc < LH_HELM_SPLIT : h->g.nvc + h->beside < LH_HELM_SPLIT_MX;
+}
+static int launch_helm_split_mx(lh_handle *h, int kRK) {
+  const Geo &g = h->g;
+  const int *iu = h->ib ? h->d_ibslot_u : nullptr, *iv = h->ib ? h->d_ibslot_v : nullptr;
+  float2 *ysf = (float2 *)h->ysf;
+  HelmMxArgs a = {{(double *)h->u1, (double *)h->u3, (double *)h->u2},
+                  {(float *)h->Nu1, (float *)h->Nu3, (float *)h->Nu2},
+                  {(float *)h->N1xz, (float *)h->N3xz, (float *)h->N2xz},
+                  {(const float *)h->uvf, (const float *)h->wvf, (const float *)h->vvc},
+                  (const double *)h->p, {ysf, ysf + 2 * (size_t)g.nu * g.ncol, (float2 *)h->ysv}, {iu, iu, iv},
+                  (const float2 *)h->duib, kRK};
+  KL("k_helm_rhs", k_helm_rhs_mx<<<dim3(3 * ((2 * g.nvc + 127) / 128), (g.nu + LH_HL - 1) / LH_HL), 128, 0, h->st>>>(a, g, h->sc));
+  KL("k_helm_sweep", k_helm_sweep_mx<<<dim3((2 * g.nvc + LH_HS_T - 1) / LH_HS_T, 3), LH_HS_T, hsweep_mx_smem(g.nu), h->st>>>(a, g, h->sc));
+  return LH_OK;
+}
 static int launch_helm_split(lh_handle *h, int kRK) {
+  if (h->prec == LH_PREC_MIXED) return launch_helm_split_mx(h, kRK);
   const Geo &g = h->g;
   const size_t n = 2 * (size_t)g.nu * g.ncol;
   const int *iu = h->ib ? h->d_ibslot_u : nullptr, *iv = h->ib ? h->d_ibslot_v : nullptr;
@@ -1834,7 +1853,9 @@ extern "C" int lh_autotune(lh_handle *h) {
   if (e != cudaSuccess) { cudaFree(save); return fail(h, LH_ECUDA, cudaGetErrorString(e)); }
   // trials: every block size with every staging depth (0: the register-prefetch kernels); each
   // solve kernel keeps the configuration of its fastest trial. The FP64 form's Helmholtz kernels
-  // depend on the block size only.
+  // depend on neither. A small channel alone takes the split routes, which have no such choices:
+  // the trials run the fused kernels, which it takes in a batch.
+  h->beside = LH_PRESS_SPLIT_COLS;
   const int cand[] = {64, 128, 256}, cpf[] = {0, 2, 4, 8};
   double best[3] = {1e30, 1e30, 1e30};
   int pick[3] = {h->tb_uw, h->tb_v, h->tb_p}, pickpf[3] = {h->pf_uw, h->pf_v, h->pf_p};
@@ -1859,6 +1880,7 @@ extern "C" int lh_autotune(lh_handle *h) {
         }
     if (copy_all(false) != cudaSuccess) rc = fail(h, LH_ECUDA, "state restore failed");
   }
+  h->beside = 0;
   cudaFree(save);
   h->tb_uw = pick[0]; h->tb_v = pick[1]; h->tb_p = pick[2];
   h->pf_uw = pickpf[0]; h->pf_v = pickpf[1]; h->pf_p = pickpf[2];

@@ -269,6 +269,9 @@ __device__ __forceinline__ void cpa4(void *dst, const void *src) {
 __device__ __forceinline__ void cpa8s(unsigned dst, const void *src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src) : "memory");
 }
+__device__ __forceinline__ void cpa4s(unsigned dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst), "l"(src) : "memory");
+}
 __device__ __forceinline__ void cpa_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cpa_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
@@ -1189,8 +1192,7 @@ __global__ void __launch_bounds__(NTHR) k_helm_v_mx3(double *__restrict__ u2, fl
 // warps a scheduler): the right-hand sides element-wise over (column, chunk of levels), then the
 // sweeps alone. An FP64 warp instruction holds its scheduler's half lane a clock for 64 cycles;
 // a fused sweep with a lane per component held 26 of them a level, alone it holds the
-// factorisation and three. (In the mixed form the same split was faster for a channel alone and
-// 6 % slower for an ensemble, whose channels fill the GPU together.) The right-hand side takes
+// factorisation and three. The right-hand side takes
 // the place of N_xz, which nothing reads after it, and the sweep's y that of the right-hand side.
 // 32 x 32 x 153, us a launch of the fused sweep u/w 165, v 164 (side by side) -> 23 + 76.
 // ============================================================================
@@ -1385,6 +1387,218 @@ __global__ void __launch_bounds__(LH_HS_T) k_helm_sweep64(HelmArgs a, Geo g, con
         ou -= ls;
       }
       h = h == ring + 2 * BE ? ring : h + BE;
+    }
+  }
+  cpa_wait<0>();
+}
+
+// ============================================================================
+// The mixed form's solves below LH_HELM_SPLIT_MX columns (of the channel and those beside it in a
+// batch): as above, the right-hand sides element-wise, then the sweeps of all three fields in one
+// launch. The operations and roundings are those of k_helm_u_mx2 / k_helm_v_mx2 (the fused
+// multiply-adds that the compiler makes of those expressions are written out), so the results
+// are the same bit for bit. The right-hand side takes the place of N_xz.
+// us a step, fused -> split, among others / alone: 32 x 32 x 153 (544 columns) 203 / 479 -> 162 / 345,
+// 64 x 64 x 129 (2112) 300 / 534 -> 301 / 466, 96 x 64 x 129 (3136) 380 / 600 -> 404 / 567,
+// 96 x 96 x 129 (4704) 511 / 722 -> 572 / 709, 128 x 128 x 201 (8320) 1257 / 1544 -> 1491 / 1695.
+// ============================================================================
+#define LH_HELM_SPLIT_MX 2432
+struct HelmMxArgs {
+  double *u[3];            // u, w, v
+  float *Nu[3];
+  float *X[3];             // N_xz, then the right-hand side
+  const float *F[3];
+  const double *p;
+  float2 *ys[3];           // y, upper factor
+  const int *ibslot[3];
+  const float2 *duib;
+  int kRK;
+};
+// grid: x = (lane block, field), y = chunk of levels
+__global__ void __launch_bounds__(128) k_helm_rhs_mx(HelmMxArgs ar, Geo g, const DevScalars *__restrict__ sc) {
+  const int f = blockIdx.x % 3, tid = (blockIdx.x / 3) * 128 + threadIdx.x, vc = tid >> 1, part = tid & 1;
+  if (vc >= g.nvc) return;
+  int c, bd;
+  vcol_of(g, vc, c, bd);
+  if (c == 0) return;  // mode (0,0): k_helm00_pcr (FP64)
+  const bool V = f == 2;
+  const int qlo = g.bq[bd][V ? 2 : 0], qhi = g.bq[bd][V ? 3 : 1], kRK = ar.kRK, nc = g.ncol;
+  const int q0 = qlo + 1 + blockIdx.y * LH_HL, q1 = min(q0 + LH_HL, qhi);
+  if (q0 >= q1) return;
+  const int r = c / g.N1h, kx = c - r * g.N1h;
+  const float k2f = (float)(g.k2x[kx] + g.k2z[r]);
+  const float C1 = (float)(g.aRK[kRK - 1] / g.Re), C2 = (float)(-g.cRK[kRK - 1]);
+  const double dR = g.dRK[kRK - 1];
+  const float G = (float)(-g.gRK[kRK - 1]);
+  const float dd = (float)g.dd, dRf = (float)dR;
+  const float dtf = (float)sc->dt, beta = (float)(g.bRK[kRK - 1] * sc->dt / g.Re);
+  const float C3u = (float)(-dR * (f ? g.k1z[r] : g.k1x[kx]));
+  const int nl = V ? g.nv : g.nu;
+  const float *d2f = V ? g.d2vf : g.d2uf, *sdgt = V ? g.sdgv : g.sdgu, *tht = V ? g.thvf : g.thuf;
+  const int *ibslot = ar.ibslot[f];
+  const size_t ls = (size_t)nc * 2, ci = (size_t)c * 2 + part;
+  const double *u = ar.u[f] + ci;
+  const float *F = ar.F[f] + ci;
+  float *Nu = ar.Nu[f] + ci, *X = ar.X[f] + ci;
+  size_t e = (size_t)q0 * ls;
+  const double um = u[e - ls];
+  double u0 = u[e];
+  float fdm = q0 == qlo + 1 ? d2f_alu(um - u0) : -d2f_alu(u0 - um);
+  float flm = V ? F[e] : F[e - ls];
+  float pm = V ? d2f_alu(ar.p[ci + e - ls]) : 0.f;
+#pragma unroll 2
+  for (int q = q0; q < q1; ++q, e += ls) {
+    const double up1 = u[e + ls];
+    const float flq = V ? F[e + ls] : F[e], nuq = Nu[e], xq = X[e];
+    const float a = d2f[q], cc = d2f[2 * nl + q], sdg = sdgt[q] + k2f, thq = tht[q];
+    const int ibs = ibslot ? ibslot[q] : -1;
+    const float fdp = d2f_alu(up1 - u0);
+    const float L = __fmaf_rn(sdg, d2f_alu(u0), __fmaf_rn(a, fdm, __fmul_rn(cc, fdp)));
+    fdm = -fdp;
+    float pt, C3;
+    if (V) {
+      const float pq = d2f_alu(ar.p[ci + e]);
+      pt = pq - pm;
+      pm = pq;
+      C3 = -dRf * dd * thq;
+    } else {
+      const double po = ar.p[((size_t)(q - 1) * nc + c) * 2 + (part ^ 1)];  // i*C3*p: (-C3 p.y, C3 p.x)
+      pt = part ? d2f_alu(po) : -d2f_alu(po);
+      C3 = C3u;
+    }
+    float du;
+    if (ibs < 0) {
+      du = __fmaf_rn(C3, pt, __fmaf_rn(C1, L, __fmul_rn(C2, nuq)));
+      const float n = __fmaf_rn(__fmul_rn(__fsub_rn(flq, flm), thq), dd, xq);
+      Nu[e] = n;
+      du = __fmaf_rn(G, n, du);
+    } else {
+      const float2 di = ar.duib[((size_t)ibs * 3 + (V ? 1 : 2 * f)) * nc + c];
+      du = part ? di.y : di.x;
+    }
+    X[e] = __fmaf_rn(beta, L, __fmul_rn(dtf, du));
+    u0 = up1;
+    flm = flq;
+  }
+}
+// The sweeps of one field: lane = (column segment, part), field blockIdx.y; the inputs of two batches
+// of U levels are on their way while one is worked on.
+__host__ __device__ constexpr int hsweep_mx_region() { return (3 * LH_HS_U * 2) | 1; }  // doubles of a thread's ring
+__host__ __device__ constexpr size_t hsweep_mx_smem(int nlev) {
+  return 8 * (size_t)LH_HS_T * hsweep_mx_region() + 4 * (size_t)3 * nlev;
+}
+__global__ void __launch_bounds__(LH_HS_T) k_helm_sweep_mx(HelmMxArgs ar, Geo g, const DevScalars *__restrict__ sc) {
+  constexpr int U = LH_HS_U;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int f = blockIdx.y, kRK = ar.kRK;
+  const bool V = f == 2;
+  const int nl = V ? g.nv : g.nu;
+  double *ring = reinterpret_cast<double *>(smem_raw) + threadIdx.x * hsweep_mx_region();
+  float *ta = reinterpret_cast<float *>(reinterpret_cast<double *>(smem_raw) + LH_HS_T * hsweep_mx_region()), *tb = ta + nl,
+        *tc = tb + nl;
+  {
+    const float *d2f = V ? g.d2vf : g.d2uf;
+    for (int i = threadIdx.x; i < nl; i += LH_HS_T) { ta[i] = d2f[i]; tb[i] = d2f[nl + i]; tc[i] = d2f[2 * nl + i]; }
+  }
+  __syncthreads();
+  const int tid = blockIdx.x * LH_HS_T + threadIdx.x, vc = tid >> 1, part = tid & 1;
+  if (vc >= g.nvc) return;
+  int c, bd;
+  vcol_of(g, vc, c, bd);
+  if (c == 0) return;
+  const int qlo = g.bq[bd][V ? 2 : 0], qhi = g.bq[bd][V ? 3 : 1];
+  const int r = c / g.N1h, kx = c - r * g.N1h;
+  const float k2f = (float)(g.k2x[kx] + g.k2z[r]);
+  const float beta = (float)(g.bRK[kRK - 1] * sc->dt / g.Re);
+  const double gw1 = g.gw[bd][0], gw2 = g.gw[bd][1];
+  const size_t ls = (size_t)g.ncol * 2, ci = (size_t)c * 2 + part;
+  double *u = ar.u[f] + ci;
+  float2 *ys = ar.ys[f] + ci;
+  const unsigned rs = (unsigned)__cvta_generic_to_shared(ring);
+  const double ulo = u[(size_t)qlo * ls], uhi = u[(size_t)qhi * ls], uhm = u[(size_t)(qhi - 1) * ls];
+  float y = V ? d2f_alu(-ulo) : d2f_alu(-(ulo + gw1 * u[(size_t)(qlo + 1) * ls]));  // first row
+  float a3raw = V ? 0.f : (float)gw1, a2p = 1.f;
+  {
+    const float *in = ar.X[f] + ci + (size_t)(qlo + 1) * ls;
+    int left = qhi - qlo - 1;
+    unsigned dst = rs;
+    auto fetch = [&]() {
+#pragma unroll
+      for (int i = 0; i < U; ++i)
+        if (left > i) { cpa4s(dst + 4 * i, in); in += ls; }
+      left -= U;
+      dst = dst == rs + 8 * U ? rs : dst + 4 * U;
+      cpa_commit();
+    };
+    fetch();
+    fetch();
+    float2 *o = ys + (size_t)qlo * ls;
+    const float *r0 = reinterpret_cast<const float *>(ring), *h = r0;
+    int q = qlo + 1;
+    for (int n = qhi - qlo - 1; n > 0; n -= U) {
+      fetch();
+      cpa_wait<2>();
+#pragma unroll
+      for (int i = 0; i < U; ++i) {
+        if (i > 0 && n <= i) break;
+        const float a = ta[q + i], b = tb[q + i], cc = tc[q + i], rr = h[i];
+        const float a1 = -beta * a;
+        const float a2 = __fmaf_rn(-beta, __fadd_rn(b, k2f), 1.f);
+        const float a3p = a3raw * a2p;
+        *o = make_float2(y, a3p);
+        o += ls;
+        a2p = 1.f / __fmaf_rn(-a1, a3p, a2);
+        y = __fmul_rn(__fmaf_rn(-a1, y, rr), a2p);
+        a3raw = -beta * cc;
+      }
+      q += U;
+      h = h == r0 + 2 * U ? r0 : h + U;
+    }
+  }
+  cpa_wait<0>();
+  {
+    const float a3p = a3raw * a2p;
+    ys[(size_t)(qhi - 1) * ls] = make_float2(y, a3p);
+    if (V) {  // last row: d(n-1) = -v(n-1)
+      y = d2f_alu(-uhi);
+    } else {  // last row: gw2 d(n-2) + d(n-1) = -(gw2 u(n-2) + u(n-1))
+      const float a1 = (float)gw2;
+      const float rl = d2f_alu(-(gw2 * uhm + uhi));
+      a2p = 1.f / (1.f - a1 * a3p);
+      y = (rl - a1 * y) * a2p;
+    }
+    u[(size_t)qhi * ls] = uhi + f2d_alu(y);
+  }
+  __threadfence();  // the copies below read what this thread stored above
+  {
+    const float2 *fy = ys + (size_t)(qhi - 1) * ls;
+    const double *fu = u + (size_t)(qhi - 1) * ls;
+    double *ou = u + (size_t)(qhi - 1) * ls;
+    int left = qhi - qlo;
+    unsigned dst = rs;
+    auto fetch = [&]() {
+#pragma unroll
+      for (int i = 0; i < U; ++i)
+        if (left > i) { cpa8s(dst + 16 * i, fy); cpa8s(dst + 16 * i + 8, fu); fy -= ls; fu -= ls; }
+      left -= U;
+      dst = dst == rs + 32 * U ? rs : dst + 16 * U;
+      cpa_commit();
+    };
+    fetch();
+    fetch();
+    const double *h = ring;
+    for (int n = qhi - qlo; n > 0; n -= U) {
+      fetch();
+      cpa_wait<2>();
+#pragma unroll
+      for (int i = 0; i < U; ++i) {
+        if (i > 0 && n <= i) break;
+        const float2 ya = reinterpret_cast<const float2 *>(h)[2 * i];
+        y = ya.x - ya.y * y;
+        *ou = h[2 * i + 1] + f2d_alu(y);
+        ou -= ls;
+      }
+      h = h == ring + 4 * U ? ring : h + 2 * U;
     }
   }
   cpa_wait<0>();

@@ -25,12 +25,16 @@ def channel(s, form, st):
     return g
 
 
-# 128 x 128 and 96 x 96: 8320 and 4704 columns; alone below 16384 (split pressure), together above it
-@pytest.mark.parametrize("form,flpress,ny", [("mixed", 0, 45), ("mixed", 1, 46), ("fp64", 0, 46), ("fp64", 1, 45)])
-def test_pressure_routes_agree(cuda_ok, form, flpress, ny):
+# 8320 and 4704 columns: alone below 16384 (split pressure), together above it; 2112, 1200 and 544:
+# alone below 2432 (split solves of the mixed form), together above it
+@pytest.mark.parametrize("form,sizes,flpress,ny,posts", [
+    ("mixed", (128, 128, 96), 0, 45, False), ("mixed", (128, 128, 96), 1, 46, False),
+    ("fp64", (128, 128, 96), 0, 46, False), ("fp64", (128, 128, 96), 1, 45, False),
+    ("mixed", (64, 48, 32), 0, 46, True), ("mixed", (64, 48, 32), 1, 45, False)])
+def test_split_and_fused_routes_agree(cuda_ok, form, sizes, flpress, ny, posts):
     alone, batched = [], []
-    for i, n in enumerate((128, 128, 96)):
-        s = build_setup(re_tau_params(n, ny + i, flpress=flpress))
+    for i, n in enumerate(sizes):
+        s = build_setup(re_tau_params(n, ny + i, flpress=flpress, posts=posts, post_period=12, post_points=6))
         st = initial_field(s, 700 + i)
         alone.append(channel(s, form, st))
         batched.append(channel(s, form, st))
