@@ -447,6 +447,14 @@ template <int N, int NL> __host__ __device__ constexpr int fx_xslots() {
 // transform. The products are formed from the integer fields, normalised by each field's
 // largest value on the line, as the forward transform's first stage reads them.
 // ============================================================================
+// bits of a product's operands: two of them give products that the forward transform has headroom
+// for (and one bit for the row separation)
+template <int N> __host__ __device__ constexpr int fx_opbits() {
+  constexpr int PBITS = 62 + fx_drop<N>() - fx_log2_up(fx_headroom<N, false>() * 1.4143f);
+  constexpr int TB = (64 + PBITS) / 2;
+  static_assert(TB <= 62, "operands of fx_mul");
+  return TB;
+}
 // Products uu, uw, vv, ww (u level) or uv, wv (v level) of the fields' lines f * PB + pb in res and
 // their forward transforms, lines p * PB + pb in res (two stages) or oth (three). One code for
 // both kinds of level: the kernel's code has to stay in the instruction cache.
@@ -457,17 +465,17 @@ __device__ __forceinline__ void fx_xpass_forward(bool isU, fx2 *res, fx2 *oth, c
   constexpr int DROP = fx_drop<N>();
   auto fa = [&](int p) { return isU ? (p > 0 ? p - 1 : 0) : 2 * p; };
   auto fb = [&](int p) { return isU ? (p == 0 ? 0 : p == 2 ? 1 : 2) : 1; };
+  // to 63 bits by the line's shift, then to TB bits
   auto shift = [](fx2 v, int l) {
-    const int a = l > 0 ? l : 0, b = l < 0 ? -l : 0;
     fx2 r;
-    r.x = (long long)((unsigned long long)v.x << a) >> b;
-    r.y = (long long)((unsigned long long)v.y << a) >> b;
+    r.x = (long long)((unsigned long long)v.x << l) >> (63 - fx_opbits<N>());
+    r.y = (long long)((unsigned long long)v.y << l) >> (63 - fx_opbits<N>());
     return r;
   };
   const int nl = (isU ? 4 : 2) * PB;
   if ((int)threadIdx.x < nl) {
     const int p = threadIdx.x / PB, pb = threadIdx.x - p * PB, a = fa(p) * PB + pb, b = fb(p) * PB + pb;
-    sP[threadIdx.x] = (fS[a] == FX_NAN || fS[b] == FX_NAN) ? FX_NAN : fS[a] + fl[a] + fS[b] + fl[b] - 64 - DROP;
+    sP[threadIdx.x] = (fS[a] == FX_NAN || fS[b] == FX_NAN) ? FX_NAN : fS[a] + fl[a] + fS[b] + fl[b] - 2 * (63 - fx_opbits<N>()) - 64 - DROP;
   }
   auto ld = [&](int line, int e) {
     const int p = line / PB, pb = line - p * PB, a = fa(p) * PB + pb, b = fb(p) * PB + pb;
@@ -527,12 +535,8 @@ __global__ void __launch_bounds__(fx_xt(N)) k_xpass_fx(const double2 *__restrict
       });
   __syncthreads();
   if (tid < NL) {
-    // |v| <= 2^(64 - clz): shifted to 2^TB, two operands of TB bits give products that the
-    // forward transform has headroom for (and one bit for the row separation)
-    constexpr int PBITS = 62 + fx_drop<N>() - fx_log2_up(fx_headroom<N, false>() * 1.4143f);
-    constexpr int TB = (64 + PBITS) / 2;
-    static_assert(TB <= 62, "operands of fx_mul");
-    fl[tid] = TB - (64 - __clz(lm[tid]));
+    // |v| <= 2^(64 - clz)
+    fl[tid] = __clz(lm[tid]) - 1;
     fS[tid] = sL[tid].S;
   }
   __syncthreads();
