@@ -667,7 +667,7 @@ extern "C" int lh_create(const lh_config *cfg, lh_handle **out) {
     h->tg.Tw = th.Tw; h->tg.T = th.T; h->tg.nx = cfg->triad_nx; h->tg.nz = cfg->triad_nz; h->tg.P = th.P;
     h->tri_nterms = th.nterms;
     h->tri_threads = std::min(32 * th.Tw, 512);
-    h->tri_smem = (size_t)(3 * th.P + 1) * h->vsz;
+    h->tri_smem = (size_t)(3 * th.P + 1 + (h->prec == LH_PREC_FP64 ? TRI_ZSLOTS : 0)) * h->vsz;
     int lim = 0;
     if (smem_optin(&lim) || h->tri_smem > (size_t)lim) {
       rc = fail(h, LH_EINVAL, "plane too large for the triad form (shared memory)"); lh_destroy(h); return rc;

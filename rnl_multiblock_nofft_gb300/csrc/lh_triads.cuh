@@ -31,8 +31,9 @@
 // uw and wu (uv and vu, vw and wv) sum the same terms with the fields' roles exchanged: the part
 // that both lists hold is summed once for both, each list's rest for itself. For complete lists
 // that leaves half of the terms, for thresholded ones what they have in common; any list gives
-// the same sum up to its order. 32 x 32 x 153, complete lists: a step 8.10 -> 4.51 ms. (The
-// mixed form keeps the lists' own order.)
+// the same sum up to its order. 32 x 32 x 153, complete lists: a step 8.10 -> 4.51 ms; with the
+// zeroth-mode sums by the whole block and the warps' order below 4.51 -> 4.24. (The mixed form
+// keeps the lists' own order.)
 #pragma once
 #include <stdint.h>
 
@@ -132,6 +133,35 @@ __device__ V tri_zeroth(const V *A, const V *Pf, int klo, int N1, int N2, int N1
   return acc;
 }
 
+#define TRI_ZSLOTS 32
+// the same by the whole block, FP64 form: 1056 terms at N 32, which on one thread held its warp (the one
+// with the longest lists) for 40 % more terms. part: a slot per warp, to be added up in order
+__device__ __forceinline__ void tri_zeroth_block(const double2 *A, const double2 *Pf, int klo, int N1, int N2, int N1h,
+                                                 double2 *part) {
+  const int nk = N2 / 2 - klo, n = (N1 + 1) * nk;
+  double2 acc = czero<double2>();
+  for (int idx = threadIdx.x; idx < n; idx += blockDim.x) {
+    const int i = idx / nk - N1 / 2, k = klo + idx % nk, ia = i < 0 ? -i : i;
+    const bool ca = i < 0, cp = -i < 0;
+    double2 a = A[tri_krow(ca ? -k : k, N2) * N1h + ia];
+    double2 p = Pf[tri_krow(cp ? k : -k, N2) * N1h + ia];
+    if (ca) a.y = -a.y;
+    if (cp) p.y = -p.y;
+    tri_mac(acc, a, p);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+    acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+  }
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+}
+__device__ __forceinline__ double2 tri_zeroth_sum(const double2 *part) {
+  double2 s = part[0];
+  for (int w = 1; w < (int)(blockDim.x >> 5); ++w) s = cadd(s, part[w]);
+  return s;
+}
+
 template <typename T>
 __device__ __forceinline__ typename C2<T>::t tri_lin(T s1, typename C2<T>::t x1, T s2, typename C2<T>::t x2) {
   typename C2<T>::t r;
@@ -149,7 +179,7 @@ __global__ void __launch_bounds__(512) k_triad(const double2 *__restrict__ u1, c
                                                typename C2<T>::t *__restrict__ vvc, typename C2<T>::t *__restrict__ wvf) {
   typedef typename C2<T>::t V;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  V *F = reinterpret_cast<V *>(smem_raw);  // [3][P] + zero slot
+  V *F = reinterpret_cast<V *>(smem_raw);  // [3][P] + zero slot (+ TRI_ZSLOTS)
   const bool isU = blockIdx.x < (unsigned)g.nuI;
   const int q = isU ? blockIdx.x + 1 : blockIdx.x - g.nuI + 1;
   const int nc = g.ncol, N1h = g.N1h, N2 = g.N2, P = tg.P;
@@ -195,8 +225,24 @@ __global__ void __launch_bounds__(512) k_triad(const double2 *__restrict__ u1, c
   const int kw = 2 * tg.nz + 1;
   const int *lid = tg.lid + (size_t)(isU ? q : g.nu + q) * 9;
   const int lane = threadIdx.x & 31;
-  // targets: (lt, kt) with list terms
-  for (int sl = threadIdx.x; sl < tg.Tw * 32; sl += blockDim.x) {
+  V *zpart = F + 3 * P + 1;  // FP64 form: two zeroth-mode sums of 16 warps
+  if constexpr (sizeof(T) == 8) {
+    if (isU) {
+      tri_zeroth_block(F1, F1, -(N2 / 2), g.N1, N2, N1h, zpart);
+    } else {
+      tri_zeroth_block(F0, F1, -(N2 / 2 - 1), g.N1, N2, N1h, zpart);
+      tri_zeroth_block(F2, F1, -(N2 / 2 - 1), g.N1, N2, N1h, zpart + 16);
+    }
+    __syncthreads();
+  }
+  auto zeroth = [&](const V *A, const V *Pf, int klo, int i) {
+    if constexpr (sizeof(T) == 8) return tri_zeroth_sum(zpart + 16 * i);
+    else return tri_zeroth(A, Pf, klo, g.N1, N2, N1h);
+  };
+  // targets: (lt, kt) with list terms. The slots' lists get shorter with the warp, and warps w, w + 4, ...
+  // share a scheduler: every second group of four is taken backwards, so that each gets as many terms.
+  const int snake = (blockDim.x & 127) == 0 ? (int)(threadIdx.x & 128) >> 7 : 0;
+  for (int sl = snake ? threadIdx.x ^ 96 : threadIdx.x; sl < tg.Tw * 32; sl += blockDim.x) {
     if (sl >= tg.T) continue;
     const int w = sl >> 5;
     const int tt = tg.tmap[sl];
@@ -211,7 +257,7 @@ __global__ void __launch_bounds__(512) k_triad(const double2 *__restrict__ u1, c
       V ww = tri_lin<T>((T)2 * c00, F2[c], (T)0, F2[c]);
       V uw = tri_lin<T>(a00, F2[c], c00, F0[c]);
       V wu = uw;
-      V vv = z0 ? tri_zeroth(F1, F1, -(N2 / 2), g.N1, N2, N1h) : tri_lin<T>((T)2 * b00, F1[c], (T)0, F1[c]);
+      V vv = z0 ? zeroth(F1, F1, -(N2 / 2), 0) : tri_lin<T>((T)2 * b00, F1[c], (T)0, F1[c]);
       if constexpr (sizeof(T) == 8) {
         tri_pairs(uu, F, tg, lid[0], lid[1], w, lane);
         tri_pairs(vv, F, tg, lid[2], lid[3], w, lane);
@@ -231,8 +277,8 @@ __global__ void __launch_bounds__(512) k_triad(const double2 *__restrict__ u1, c
       // F0 = u (interpolated), F1 = v, F2 = w (interpolated); lists 2 uv, 4 vu, 6 vw, 8 wv
       V vu = tri_lin<T>(a00, F1[c], b00, F0[c]);
       V vw = tri_lin<T>(b00, F2[c], c00, F1[c]);
-      V uv = z0 ? tri_zeroth(F0, F1, -(N2 / 2 - 1), g.N1, N2, N1h) : vu;
-      V wv = z0 ? tri_zeroth(F2, F1, -(N2 / 2 - 1), g.N1, N2, N1h) : vw;
+      V uv = z0 ? zeroth(F0, F1, -(N2 / 2 - 1), 0) : vu;
+      V wv = z0 ? zeroth(F2, F1, -(N2 / 2 - 1), 1) : vw;
       if constexpr (sizeof(T) == 8) {
         tri_both(uv, vu, F, tg, lid, w, lane);
         tri_both(vw, wv, F, tg, lid + 3, w, lane);
