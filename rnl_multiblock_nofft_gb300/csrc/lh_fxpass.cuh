@@ -6,10 +6,12 @@
 //
 // Measured at 256 x 256 x 301 with posts (transforms of 384), ms per step (three launches),
 // against the FP64 Stockham passes that they replaced (FP64 pipe 85 % busy, DRAM 2-5 %):
-//   inverse z 18.52 -> 4.98, x 62.94 -> 15.37, forward z 19.01 -> 6.50, immersed-boundary
-//   x round trip 6.58 -> 1.76, its z transforms 1.95 -> 0.51 and 2.04 -> 0.54; the whole
-//   step 123.4 -> 39.2 (6.20, 16.85, 7.39 and 43.0 with two FP64 additions per converted
-//   result, which kept the FP64 pipe 57-74 % busy). Instruction issue bounds them now.
+//   inverse z 18.52 -> 4.74, x 62.94 -> 15.30, forward z 19.01 -> 5.76, immersed-boundary
+//   x round trip 6.58 -> 1.68, its z transforms 1.95 -> 0.49 and 2.04 -> 0.59; the whole
+//   step 123.4 -> 38.7 (6.20, 16.85, 7.39 and 43.0 with two FP64 additions per converted
+//   result, which kept the FP64 pipe 57-74 % busy). The x pass issues on 52 % of the cycles
+//   (ALU 45 %, FP64 26 %) and waits on barriers and instruction fetch; the forward z pass
+//   waits on its conversions (FP64 56 %) and on shared memory.
 #pragma once
 #include "lh_fx.cuh"
 #include "lh_kernels.cuh"

@@ -10,15 +10,16 @@
 //   k_zfwd_fx, k_zfwd2  : forward z transforms (cft, iopt<0) + der_x/der_z (FOU3D.f90:476-593):
 //                 N_xz of u, v, w and the y-flux products uv, vv, wv
 //   k_dt        : dt = min(2.5 dtv, CFL dtc) on the device (FOU3D.f90:291-297)
-//   k_helm_uw   : RHS0_u1/u3 + der_yu_h + du += -gRK N + solveU_W, one thread per column
-//   k_helm_v    : RHS0_u2 + der_yv_h + du += -gRK N + solveV
+//   k_helm64    : RHS0 + der_y_h + du += -gRK N + solveU_W / solveV of the FP64 form, both parts of
+//                 a column in a lane; channels of few columns: k_helm_rhs, k_helm_sweep64
 //   k_meanflow  : flowrate_corr on mode (0,0) (constant flow rate)
 //   k_press3 (k_press2), or k_press_rhs, k_press_sweep, k_press_corr : divergence + solveP (LUsolP with the stored factors, k_build_dg) + v_corr
 //                 + divergence of the corrected field in the third substep (max |div| -> err)
 //   k_ib_du(_mx), k_spec_zinv(_fx, 2), k_ib_xforce(_fx), k_zfwd_spec(_fx, 2) : immersed-boundary
 //                 forcing of du (imm_bounds_u/v, FOU3D.f90:806-998) when the geometry has posts
-//   Mixed form (LH_PREC_MIXED): FP32 transforms, and k_helm_u_mx2 / k_helm_v_mx2 solve
-//   the Helmholtz systems for the increment in FP32 on top of the FP64 state.
+//   Mixed form (LH_PREC_MIXED): FP32 transforms, and k_helm_u_mx2 / k_helm_v_mx2 (staged: _mx3; few
+//   columns: k_helm_rhs_mx, k_helm_sweep_mx) solve the Helmholtz systems for the increment in FP32
+//   on top of the FP64 state.
 // On request: k_xstats, k_wx_stats, k_spectra, k_slip (statistics), k_band_io, k_transpose
 // (state I/O).
 #pragma once
