@@ -2152,6 +2152,9 @@ __global__ void __launch_bounds__(NTHR) k_press3(double *__restrict__ u1, double
 // ============================================================================
 #define LH_PRESS_SPLIT_COLS 16384
 #define LH_PL 8  // levels of a thread of the element-wise kernels (rolling v, psi)
+__host__ __forceinline__ int press_chunks(const Geo &g) { return (g.np + LH_PL - 1) / LH_PL; }
+// the third substep's faces below the chunks, [chunk][segment]
+__host__ __forceinline__ size_t press_faces_bytes(const Geo &g) { return sizeof(double2) * press_chunks(g) * (size_t)g.nvc; }
 // a b + c d + t dv with the roundings of k_press3's compiled expression (the fused operations are
 // written out throughout, so that both routes of the pressure step agree bit for bit)
 __device__ __forceinline__ double press_div(double a, double b, double c, double d, double t, double dv) {

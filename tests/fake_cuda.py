@@ -1,0 +1,34 @@
+"""Runs a channel's host code without a GPU, on the stand-in runtime of tests/fake_cudart.c, and
+reads its log."""
+import os
+import subprocess
+import sys
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+
+
+def build(tmp):
+    so = str(tmp / "libfake_cudart.so")
+    subprocess.run(["gcc", "-std=gnu11", "-O1", "-Wall", "-Werror", "-fPIC", "-shared",
+                    os.path.join(HERE, "fake_cudart.c"), "-o", so], check=True)
+    return so
+
+
+def run(so, log, code, args=""):
+    """Runs `code` in a process of its own; returns (its standard output, the log's lines as lists)"""
+    env = dict(os.environ, LD_PRELOAD=so, FAKE_CUDART_LOG=str(log), FAKE_CUDART_ARGS=args, PYTHONPATH=ROOT)
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-3000:]
+    return r.stdout, [l.split() for l in open(log)]
+
+
+def allocations(lines):
+    """[(first byte, bytes)] of the device arrays"""
+    return [(int(l[1], 16), int(l[2])) for l in lines if l[0] == "A"]
+
+
+def launches(lines, kernel):
+    """[(position in the log, grid, [arguments])] of the launches whose name contains `kernel`"""
+    return [(i, tuple(int(x) for x in l[3:6]), [0 if x == "(nil)" else int(x, 16) for x in l[10:]])
+            for i, l in enumerate(lines) if l[0] == "L" and kernel in l[1]]
