@@ -1421,7 +1421,7 @@ static int substep_launches_t(lh_handle *h, int kRK) {
   }
   if (fork) CK(cudaStreamWaitEvent(h->st, h->ev_join, 0));
   // otherwise the mean-flow correction follows the join: beside the pressure's right-hand side and
-  // sweep where these are launches of their own (they read u(0,0) times k = 0), else before. (Large
+  // sweep where these are launches of their own (k_press_rhs leaves u(0,0) unread), else before. (Large
   // channels fill the GPU: beside their solves it cost a step 0.8 %.)
   if (!(mixed00 && fork && split)) {
     const bool beside = fork && split;

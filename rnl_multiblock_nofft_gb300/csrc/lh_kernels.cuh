@@ -2161,7 +2161,9 @@ __device__ __forceinline__ double press_div(double a, double b, double c, double
   return __fma_rn(t, dv, __fma_rn(a, b, __dmul_rn(c, d)));
 }
 // psi = dti/(a+b) div: thread = (column segment, chunk), both parts; vlow (third substep): the face
-// below each chunk, [chunk][segment], for the corrections' divergence
+// below each chunk, [chunk][segment], for the corrections' divergence. u and w of mode (0,0), whose
+// factors are zero, are not read (v is, in their place): the mean-flow correction may be writing u(0,0)
+// beside this kernel.
 __global__ void __launch_bounds__(128) k_press_rhs(const double2 *__restrict__ u1, const double2 *__restrict__ u2,
                                                    const double2 *__restrict__ u3, double2 *__restrict__ psi,
                                                    double2 *__restrict__ vlow, Geo g, const DevScalars *__restrict__ sc,
@@ -2176,6 +2178,7 @@ __global__ void __launch_bounds__(128) k_press_rhs(const double2 *__restrict__ u
   const int nc = g.ncol, r = c / g.N1h, kx = c - r * g.N1h;
   const double dtirk = sc->dti / (g.aRK[kRK - 1] + g.bRK[kRK - 1]);
   const double dkx = dtirk * g.k1x[kx], dkz = dtirk * g.k1z[r];
+  const double2 *uc = c != 0 ? u1 : u2, *wc = c != 0 ? u3 : u2;
   double2 vm = u2[(size_t)q0 * nc + c];
   if (vlow) vlow[(size_t)blockIdx.y * g.nvc + vc] = vm;
 #pragma unroll
@@ -2183,7 +2186,7 @@ __global__ void __launch_bounds__(128) k_press_rhs(const double2 *__restrict__ u
     const int qp = q0 + i;
     if (qp > phi) break;
     const size_t e = (size_t)(qp + 1) * nc + c;
-    const double2 a = u1[e], w = u3[e], v = u2[e];
+    const double2 a = uc[e], w = wc[e], v = u2[e];
     const double th = dtirk * g.thud[qp + 1];
     double2 rhs;
     rhs.x = press_div(-dkx, a.y, -dkz, w.y, th, v.x - vm.x);

@@ -32,3 +32,20 @@ def launches(lines, kernel):
     """[(position in the log, grid, [arguments])] of the launches whose name contains `kernel`"""
     return [(i, tuple(int(x) for x in l[3:6]), [0 if x == "(nil)" else int(x, 16) for x in l[10:]])
             for i, l in enumerate(lines) if l[0] == "L" and kernel in l[1]]
+
+
+def concurrent(lines, kernel):
+    """The kernels that no stream order or event orders against a launch whose name contains `kernel`"""
+    on, at, before = {}, {}, []  # launches that a stream's next one / an event's waiters follow; per launch
+    names = []
+    for l in lines:
+        if l[0] == "L":
+            names.append(l[1])
+            before.append(frozenset(on.get(l[2], ())))
+            on[l[2]] = before[-1] | {len(names) - 1}
+        elif l[0] == "R":
+            at[l[1]] = on.get(l[2], frozenset())
+        elif l[0] == "W":
+            on[l[1]] = on.get(l[1], frozenset()) | at.get(l[2], frozenset())
+    mine = [i for i, n in enumerate(names) if kernel in n]
+    return mine, {names[j] for i in mine for j in range(len(names)) if j != i and j not in before[i] and i not in before[j]}
