@@ -651,6 +651,18 @@ __global__ void __launch_bounds__(512) k_helm00_pcr(double *__restrict__ u1, dou
 
 
 // ============================================================================
+// The sums of products of a level, for every kernel that solves for the mixed form. Which product of
+// a b + c d is rounded would be the compiler's choice, and it chose otherwise in one of the kernels
+// (k_helm_v_mx2: 1 value in 300 off by a rounding); written out, all give the same bits.
+__device__ __forceinline__ float mx_lap(float a, float fdm, float c, float fdp, float sdg, float u) {
+  return __fmaf_rn(sdg, u, __fmaf_rn(a, fdm, __fmul_rn(c, fdp)));
+}
+__device__ __forceinline__ float mx_du(float C1, float L, float C2, float nu, float C3, float pt) {
+  return __fmaf_rn(C3, pt, __fmaf_rn(C1, L, __fmul_rn(C2, nu)));
+}
+__device__ __forceinline__ float mx_rhs(float beta, float L, float dt, float du) { return __fmaf_rn(beta, L, __fmul_rn(dt, du)); }
+
+// ============================================================================
 // Mixed-form solves with one lane per (column, real/imaginary part): the matrix
 // is real, so the two parts are independent systems; each lane repeats the FP32
 // factorisation. Scalar views: element (q, col, part) at (q*ncol + col)*2 + part.
@@ -737,12 +749,12 @@ __global__ void __launch_bounds__(NTHR) k_helm_u_mx2(double *__restrict__ u1, do
       const double po = fp[s_];
       if (q + D <= qhi - 1) HU_FETCH(s_, q + D)
       const float fdp = d2f_alu(up1 - u0);
-      const float L = a * fdm + cc * fdp + sdg * d2f_alu(u0);
+      const float L = mx_lap(a, fdm, cc, fdp, sdg, d2f_alu(u0));
       fdm = -fdp;
       float du;
       if (ibs < 0) {
         const float pt = part ? d2f_alu(po) : -d2f_alu(po);
-        du = (C1 * L + C2 * nuq) + C3 * pt;
+        du = mx_du(C1, L, C2, nuq, C3, pt);
         const float n = xq + (flq - flm) * thq * dd;
         Nu[e] = n;
         du += G * n;
@@ -750,7 +762,7 @@ __global__ void __launch_bounds__(NTHR) k_helm_u_mx2(double *__restrict__ u1, do
         const float2 di = duib[((size_t)ibs * 3 + (fw ? 2 : 0)) * nc + c];
         du = part ? di.y : di.x;
       }
-      const float rr = dtf * du + beta * L;
+      const float rr = mx_rhs(beta, L, dtf, du);
       const float a1 = -beta * a;
       const float a2 = 1.f - beta * (b + k2f);
       const float a3p = a3raw * a2p;
@@ -773,14 +785,14 @@ __global__ void __launch_bounds__(NTHR) k_helm_u_mx2(double *__restrict__ u1, do
     const float a = g.d2uf[q], b = g.d2uf[nu + q], cc = g.d2uf[2 * nu + q];
     const float sdg = g.sdgu[q] + k2f;
     const float fdp = d2f_alu(up1 - u0);
-    const float L = a * fdm + cc * fdp + sdg * d2f_alu(u0);
+    const float L = mx_lap(a, fdm, cc, fdp, sdg, d2f_alu(u0));
     fdm = -fdp;
     float du;
     const int ibs = ibslot_u ? ibslot_u[q] : -1;
     if (ibs < 0) {
       const double2 pj = p[(size_t)(q - 1) * nc + c];
       const float pt = part ? d2f_alu(pj.x) : -d2f_alu(pj.y);  // i*C3*p: (-C3 p.y, C3 p.x)
-      du = (C1 * L + C2 * Nu[e]) + C3 * pt;
+      du = mx_du(C1, L, C2, Nu[e], C3, pt);
       const float n = X[e] + (flq - flm) * g.thuf[q] * dd;
       Nu[e] = n;
       du += G * n;
@@ -788,7 +800,7 @@ __global__ void __launch_bounds__(NTHR) k_helm_u_mx2(double *__restrict__ u1, do
       const float2 di = duib[((size_t)ibs * 3 + (fw ? 2 : 0)) * nc + c];
       du = part ? di.y : di.x;
     }
-    const float rr = dtf * du + beta * L;
+    const float rr = mx_rhs(beta, L, dtf, du);
     const float a1 = -beta * a;
     const float a2 = 1.f - beta * (b + k2f);
     const float a3p = a3raw * a2p;
@@ -878,12 +890,12 @@ __global__ void __launch_bounds__(NTHR) k_helm_v_mx2(double *__restrict__ u2, fl
       const int ibs = fib[s_];
       if (q + D <= qhi - 1) HV_FETCH(s_, q + D)
       const float fdp = d2f_alu(vp1 - v0);
-      const float L = a * fdm + cc * fdp + sdg * d2f_alu(v0);
+      const float L = mx_lap(a, fdm, cc, fdp, sdg, d2f_alu(v0));
       fdm = -fdp;
       float du;
       if (ibs < 0) {
         const float C3 = -dRf * dd * thq;
-        du = (C1 * L + C2 * nuq) + C3 * pd;
+        du = mx_du(C1, L, C2, nuq, C3, pd);
         const float n = xq + (vvp - vvq) * thq * dd;
         Nu2[e] = n;
         du += G * n;
@@ -891,7 +903,7 @@ __global__ void __launch_bounds__(NTHR) k_helm_v_mx2(double *__restrict__ u2, fl
         const float2 di = duib[((size_t)ibs * 3 + 1) * nc + c];
         du = part ? di.y : di.x;
       }
-      const float rr = dtf * du + beta * L;
+      const float rr = mx_rhs(beta, L, dtf, du);
       const float a1 = -beta * a;
       const float a2 = 1.f - beta * (b + k2f);
       const float a3p = a3raw * a2p;
@@ -1035,12 +1047,12 @@ __global__ void __launch_bounds__(NTHR) k_helm_u_mx3(double *__restrict__ u1, do
     const float a = ta[q], b = tb[q], cc = tc[q], sdg = tsd[q] + k2f, thq = tth[q];
     const int ibs = tib[q];
     const float fdp = d2f_alu(up1 - u0);
-    const float L = a * fdm + cc * fdp + sdg * d2f_alu(u0);
+    const float L = mx_lap(a, fdm, cc, fdp, sdg, d2f_alu(u0));
     fdm = -fdp;
     float du;
     if (ibs < 0) {
       const float pt = part ? d2f_alu(po) : -d2f_alu(po);
-      du = (C1 * L + C2 * nuq) + C3 * pt;
+      du = mx_du(C1, L, C2, nuq, C3, pt);
       const float n = xq + (flq - flm) * thq * dd;
       Nu[e] = n;
       du += G * n;
@@ -1048,7 +1060,7 @@ __global__ void __launch_bounds__(NTHR) k_helm_u_mx3(double *__restrict__ u1, do
       const float2 di = duib[((size_t)ibs * 3 + (fw ? 2 : 0)) * nc + c];
       du = part ? di.y : di.x;
     }
-    const float rr = dtf * du + beta * L;
+    const float rr = mx_rhs(beta, L, dtf, du);
     const float a1 = -beta * a;
     const float a2 = 1.f - beta * (b + k2f);
     const float a3p = a3raw * a2p;
@@ -1152,12 +1164,12 @@ __global__ void __launch_bounds__(NTHR) k_helm_v_mx3(double *__restrict__ u2, fl
     const float pd = pq - pprev;
     pprev = pq;
     const float fdp = d2f_alu(vp1 - v0);
-    const float L = a * fdm + cc * fdp + sdg * d2f_alu(v0);
+    const float L = mx_lap(a, fdm, cc, fdp, sdg, d2f_alu(v0));
     fdm = -fdp;
     float du;
     if (ibs < 0) {
       const float C3 = -dRf * dd * thq;
-      du = (C1 * L + C2 * nuq) + C3 * pd;
+      du = mx_du(C1, L, C2, nuq, C3, pd);
       const float n = xq + (vvp - vvq) * thq * dd;
       Nu2[e] = n;
       du += G * n;
@@ -1165,7 +1177,7 @@ __global__ void __launch_bounds__(NTHR) k_helm_v_mx3(double *__restrict__ u2, fl
       const float2 di = duib[((size_t)ibs * 3 + 1) * nc + c];
       du = part ? di.y : di.x;
     }
-    const float rr = dtf * du + beta * L;
+    const float rr = mx_rhs(beta, L, dtf, du);
     const float a1 = -beta * a;
     const float a2 = 1.f - beta * (b + k2f);
     const float a3p = a3raw * a2p;
@@ -1397,8 +1409,8 @@ __global__ void __launch_bounds__(LH_HS_T) k_helm_sweep64(HelmArgs a, Geo g, con
 // The mixed form's solves below LH_HELM_SPLIT_MX columns (of the channel and those beside it in a
 // batch): as above, the right-hand sides element-wise, then the sweeps of all three fields in one
 // launch. The operations and roundings are those of k_helm_u_mx2 / k_helm_v_mx2 (the fused
-// multiply-adds that the compiler makes of those expressions are written out), so the results
-// are the same bit for bit. The right-hand side takes the place of N_xz.
+// multiply-adds are written out), so the results are the same bit for bit. The right-hand side
+// takes the place of N_xz.
 // us a step, fused -> split, among others / alone: 32 x 32 x 153 (544 columns) 203 / 479 -> 162 / 345,
 // 64 x 64 x 129 (2112) 300 / 534 -> 301 / 466, 96 x 64 x 129 (3136) 380 / 600 -> 404 / 567,
 // 96 x 96 x 129 (4704) 511 / 722 -> 572 / 709, 128 x 128 x 201 (8320) 1257 / 1544 -> 1491 / 1695.
@@ -1454,7 +1466,7 @@ __global__ void __launch_bounds__(128) k_helm_rhs_mx(HelmMxArgs ar, Geo g, const
     const float a = d2f[q], cc = d2f[2 * nl + q], sdg = sdgt[q] + k2f, thq = tht[q];
     const int ibs = ibslot ? ibslot[q] : -1;
     const float fdp = d2f_alu(up1 - u0);
-    const float L = __fmaf_rn(sdg, d2f_alu(u0), __fmaf_rn(a, fdm, __fmul_rn(cc, fdp)));
+    const float L = mx_lap(a, fdm, cc, fdp, sdg, d2f_alu(u0));
     fdm = -fdp;
     float pt, C3;
     if (V) {
@@ -1469,7 +1481,7 @@ __global__ void __launch_bounds__(128) k_helm_rhs_mx(HelmMxArgs ar, Geo g, const
     }
     float du;
     if (ibs < 0) {
-      du = __fmaf_rn(C3, pt, __fmaf_rn(C1, L, __fmul_rn(C2, nuq)));
+      du = mx_du(C1, L, C2, nuq, C3, pt);
       const float n = __fmaf_rn(__fmul_rn(__fsub_rn(flq, flm), thq), dd, xq);
       Nu[e] = n;
       du = __fmaf_rn(G, n, du);
@@ -1477,7 +1489,7 @@ __global__ void __launch_bounds__(128) k_helm_rhs_mx(HelmMxArgs ar, Geo g, const
       const float2 di = ar.duib[((size_t)ibs * 3 + (V ? 1 : 2 * f)) * nc + c];
       du = part ? di.y : di.x;
     }
-    X[e] = __fmaf_rn(beta, L, __fmul_rn(dtf, du));
+    X[e] = mx_rhs(beta, L, dtf, du);
     u0 = up1;
     flm = flq;
   }
@@ -1821,6 +1833,12 @@ __global__ void __launch_bounds__(NTHR) k_build_dg(double *__restrict__ dg1, dou
   dg3[(size_t)phi * nc + c] = 0.0;
 }
 
+// a b + c d + t dv, the sum of both routes of the pressure step: written out, as the compiler's choice of
+// the product to round need not be the same in each kernel (they agree bit for bit)
+__device__ __forceinline__ double press_div(double a, double b, double c, double d, double t, double dv) {
+  return __fma_rn(t, dv, __fma_rn(a, b, __dmul_rn(c, d)));
+}
+
 // ============================================================================
 // Pressure: divergence, psi = dti/(a+b) div (gauge on (0,0)), LUsolP with the
 // stored factors, p += psi, v_corr, and the divergence of the corrected field
@@ -1896,7 +1914,7 @@ __global__ void __launch_bounds__(NTHR, LH_PRESS_MINB) k_press2(double *__restri
           const double ao = fa[s_], wo = fw[s_], v = fv[s_], A1 = f1[s_], a2p = f2[s_];
           const double th = ft[s_];
           if (qp + D <= phi) HP_FETCH(s_, qp + D)
-          double rhs = (dskx * ao + dskz * wo) + th * (v - vm);
+          double rhs = press_div(dskx, ao, dskz, wo, th, v - vm);
           vm = v;
           if (qp == plo && c == 0 && bd == 1) rhs = 0.0;
           y = (qp == plo) ? rhs * a2p : (rhs - A1 * y) * a2p;
@@ -1950,9 +1968,9 @@ __global__ void __launch_bounds__(NTHR, LH_PRESS_MINB) k_press2(double *__restri
           const double ao = __shfl_xor_sync(pm, a, 1), wo = __shfl_xor_sync(pm, w, 1);
           if (need_div && qp < phi) {
             const double th = thu1;
-            const double dvp = (skx * aup_o + skz * wup_o) + th * (vup - v);
-            const double d2 = dvp * dvp;
-            bits_max(dmax, d2 + __shfl_xor_sync(pm, d2, 1));
+            const double dvp = press_div(skx, aup_o, skz, wup_o, th, vup - v);
+            const double d2 = __dmul_rn(dvp, dvp);
+            bits_max(dmax, __dadd_rn(d2, __shfl_xor_sync(pm, d2, 1)));
           }
           aup_o = ao; wup_o = wo; vup = v;
           xn = x;
@@ -1965,9 +1983,9 @@ __global__ void __launch_bounds__(NTHR, LH_PRESS_MINB) k_press2(double *__restri
     if (need_div) {
       const double th = g.thud[plo + 1];
       const double vb = u2[(size_t)plo * ls + ci];
-      const double dvp = (skx * aup_o + skz * wup_o) + th * (vup - vb);
-      const double d2 = dvp * dvp;
-      bits_max(dmax, d2 + __shfl_xor_sync(pm, d2, 1));
+      const double dvp = press_div(skx, aup_o, skz, wup_o, th, vup - vb);
+      const double d2 = __dmul_rn(dvp, dvp);
+      bits_max(dmax, __dadd_rn(d2, __shfl_xor_sync(pm, d2, 1)));
     }
     if (bd <= 1) {
       u1[(size_t)ulo * ls + ci] = g.gwbc1 * u1[(size_t)(ulo + 1) * ls + ci];
@@ -2054,7 +2072,7 @@ __global__ void __launch_bounds__(NTHR) k_press3(double *__restrict__ u1, double
       const double th = ptab[qp + 1];
       if (qp + D <= phi) fetch_f(qp + D);
       cpa_commit();
-      double rhs = (dskx * ao + dskz * wo) + th * (v - vm);
+      double rhs = press_div(dskx, ao, dskz, wo, th, v - vm);
       vm = v;
       if (qp == plo && c == 0 && bd == 1) rhs = 0.0;
       y = (qp == plo) ? rhs * a2p : (rhs - A1 * y) * a2p;
@@ -2102,9 +2120,9 @@ __global__ void __launch_bounds__(NTHR) k_press3(double *__restrict__ u1, double
       }
       const double ao = __shfl_xor_sync(pm, a, 1), wo = __shfl_xor_sync(pm, w, 1);
       if (need_div && qp < phi) {
-        const double dvp = (skx * aup_o + skz * wup_o) + thu1 * (vup - v);
-        const double d2 = dvp * dvp;
-        bits_max(dmax, d2 + __shfl_xor_sync(pm, d2, 1));
+        const double dvp = press_div(skx, aup_o, skz, wup_o, thu1, vup - v);
+        const double d2 = __dmul_rn(dvp, dvp);
+        bits_max(dmax, __dadd_rn(d2, __shfl_xor_sync(pm, d2, 1)));
       }
       aup_o = ao; wup_o = wo; vup = v;
       xn = x;
@@ -2113,9 +2131,9 @@ __global__ void __launch_bounds__(NTHR) k_press3(double *__restrict__ u1, double
     if (need_div) {
       const double th = g.thud[plo + 1];
       const double vb = u2[(size_t)plo * ls + ci];
-      const double dvp = (skx * aup_o + skz * wup_o) + th * (vup - vb);
-      const double d2 = dvp * dvp;
-      bits_max(dmax, d2 + __shfl_xor_sync(pm, d2, 1));
+      const double dvp = press_div(skx, aup_o, skz, wup_o, th, vup - vb);
+      const double d2 = __dmul_rn(dvp, dvp);
+      bits_max(dmax, __dadd_rn(d2, __shfl_xor_sync(pm, d2, 1)));
     }
     if (bd <= 1) {
       u1[(size_t)ulo * ls + ci] = g.gwbc1 * u1[(size_t)(ulo + 1) * ls + ci];
@@ -2155,11 +2173,6 @@ __global__ void __launch_bounds__(NTHR) k_press3(double *__restrict__ u1, double
 __host__ __forceinline__ int press_chunks(const Geo &g) { return (g.np + LH_PL - 1) / LH_PL; }
 // the third substep's faces below the chunks, [chunk][segment]
 __host__ __forceinline__ size_t press_faces_bytes(const Geo &g) { return sizeof(double2) * press_chunks(g) * (size_t)g.nvc; }
-// a b + c d + t dv with the roundings of k_press3's compiled expression (the fused operations are
-// written out throughout, so that both routes of the pressure step agree bit for bit)
-__device__ __forceinline__ double press_div(double a, double b, double c, double d, double t, double dv) {
-  return __fma_rn(t, dv, __fma_rn(a, b, __dmul_rn(c, d)));
-}
 // psi = dti/(a+b) div: thread = (column segment, chunk), both parts; vlow (third substep): the face
 // below each chunk, [chunk][segment], for the corrections' divergence. u and w of mode (0,0), whose
 // factors are zero, are not read (v is, in their place): the mean-flow correction may be writing u(0,0)
