@@ -222,8 +222,8 @@ static cudaError_t set_attrs_sized(int lim) {
   }
   if constexpr (sizeof(T) == 4) {  // the two-stage mixed-form passes
     // k_xstats also holds a small static reduction array
-    if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)k_xstats<T, N>, A, lim - 1024);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)k_ib_xforce<T, N>, A, lim);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)k_xstats<N>, A, lim - 1024);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)k_ib_xforce<N>, A, lim);
     if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)k_zinv2<N>, A, lim);
     if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)k_zfwd2<N>, A, lim);
     if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)k_spec_zinv2<N>, A, lim);
@@ -1214,7 +1214,7 @@ static int launch_ib_xforce(lh_handle *h, int npl) {
   if constexpr (sizeof(T) == 4) {
     constexpr int PB = 4 * pb_xpass<float2>(N);
     dim3 g2((h->g.G2 / 2 + PB - 1) / PB, npl);
-    KL("k_ib_xforce", k_ib_xforce<float, N><<<g2, NTHR_H, 2 * (size_t)PB * N * sizeof(float2), h->st>>>(
+    KL("k_ib_xforce", k_ib_xforce<N><<<g2, NTHR_H, 2 * (size_t)PB * N * sizeof(float2), h->st>>>(
                           (const float2 *)h->A, (float2 *)h->B, h->g, (const float2 *)h->twx, h->d_ibrec, h->d_iboff, (const float *)h->cap, h->sc));
   } else {  // FP64: fixed point
     constexpr int PB = fx_pbl(N);
@@ -1544,7 +1544,7 @@ static int launch_xstats(lh_handle *h, const Geo &g, int nslots, const void *twx
   if constexpr (sizeof(T) == 4) {
     constexpr int PB = pb_xpass<float2>(N);
     dim3 grid((g.G2 / 2 + PB - 1) / PB, nslots);
-    KL("k_xstats", k_xstats<T, N><<<grid, NTHR_H, 8 * (size_t)PB * N * sizeof(float2), h->st>>>(
+    KL("k_xstats", k_xstats<N><<<grid, NTHR_H, 8 * (size_t)PB * N * sizeof(float2), h->st>>>(
                        (const float2 *)h->A, g, (const float2 *)twx, h->st_pl, h->st_cd, h->st_ncl, h->st_dnx, h->st_dnz,
                        h->st_ntx));
   } else {  // FP64: fixed point

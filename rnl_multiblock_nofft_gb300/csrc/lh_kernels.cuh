@@ -180,11 +180,12 @@ __device__ __forceinline__ void xstats_sums(const V *__restrict__ res, const Geo
   }
 }
 
-template <typename T, int N>
-__global__ void __launch_bounds__(NTHR) k_xstats(const typename C2<T>::t *__restrict__ A, Geo g,
-                                                 const typename C2<T>::t *__restrict__ twx, double *__restrict__ pl,
-                                                 double *__restrict__ cd, int ncl, int dnx, int dnz, int ntx) {
-  typedef typename C2<T>::t V;
+// mixed form (FP64 form: k_xstats_fx)
+template <int N>
+__global__ void __launch_bounds__(NTHR) k_xstats(const float2 *__restrict__ A, Geo g, const float2 *__restrict__ twx,
+                                                 double *__restrict__ pl, double *__restrict__ cd, int ncl, int dnx,
+                                                 int dnz, int ntx) {
+  typedef float2 V;
   constexpr int PB = pb_xpass<V>(N);
   constexpr int G1 = N, H = N / 2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1239,45 +1240,45 @@ __device__ __forceinline__ void helm_rhs_field(const HelmArgs &a, const Geo &g, 
   double2 fl = V ? F[e] : F[e - nc];
   double2 pm;
   if (V) pm = a.p[e - nc];
-      const double unit = -dt / g.Re * g.aRK[kRK - 1], k2 = g.k2x[kx] + g.k2z[r];
-      const double c2 = -dt * g.cRK[kRK - 1], cg = -dt * g.gRK[kRK - 1], cp = -dt * dR;
-      const double ck = V ? 0.0 : cp * (f ? g.k1z[r] : g.k1x[kx]);
-      const double mp = (f == 0 && c == 0) ? cp * sc->mpgx : 0.0;  // u only, real part
-      const double *d2 = V ? g.d2v : g.d2u, *th = V ? g.thv : g.thu;
-  #pragma unroll 2
-      for (int q = q0; q < q1; ++q, e += nc) {
-        const double2 up1 = u[e + nc], pq = a.p[V ? e : e - nc];
-        const double2 fq = V ? F[e + nc] : F[e], nuq = Nu[e], xq = X[e];
-        const double l1 = unit * d2[q], l2 = unit * (d2[nl + q] + k2), l3 = unit * d2[2 * nl + q], thq = th[q] * g.dd;
-        const int ibs = ibslot ? ibslot[q] : -1;
-        double2 rr, nn;
-  #pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          const double upt = t ? up1.y : up1.x, u0t = t ? u0.y : u0.x, umt = t ? um.y : um.x;
-          const double flq = t ? fq.y : fq.x, flm = t ? fl.y : fl.x, nu = t ? nuq.y : nuq.x, x = t ? xq.y : xq.x;
-          double v;
-          if (ibs < 0) {
-            const double n = x + (flq - flm) * thq;
-            (t ? nn.y : nn.x) = n;
-            v = c2 * nu - (l1 * umt + (l2 * u0t + l3 * upt));  // the increment first: u's rounding enters once
-            v += cg * n;
-            if (V) {
-              v += (cp * thq) * (t ? pq.y - pm.y : pq.x - pm.x);
-            } else {
-              v += t ? ck * pq.x : -ck * pq.y;
-              if (t == 0) v += mp;
-            }
-          } else {
-            const double2 di = a.duib[((size_t)ibs * 3 + fd) * nc + c];
-            v = dt * (t ? di.y : di.x);
-          }
-          (t ? rr.y : rr.x) = u0t + v;
+  const double unit = -dt / g.Re * g.aRK[kRK - 1], k2 = g.k2x[kx] + g.k2z[r];
+  const double c2 = -dt * g.cRK[kRK - 1], cg = -dt * g.gRK[kRK - 1], cp = -dt * dR;
+  const double ck = V ? 0.0 : cp * (f ? g.k1z[r] : g.k1x[kx]);
+  const double mp = (f == 0 && c == 0) ? cp * sc->mpgx : 0.0;  // u only, real part
+  const double *d2 = V ? g.d2v : g.d2u, *th = V ? g.thv : g.thu;
+#pragma unroll 2
+  for (int q = q0; q < q1; ++q, e += nc) {
+    const double2 up1 = u[e + nc], pq = a.p[V ? e : e - nc];
+    const double2 fq = V ? F[e + nc] : F[e], nuq = Nu[e], xq = X[e];
+    const double l1 = unit * d2[q], l2 = unit * (d2[nl + q] + k2), l3 = unit * d2[2 * nl + q], thq = th[q] * g.dd;
+    const int ibs = ibslot ? ibslot[q] : -1;
+    double2 rr, nn;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      const double upt = t ? up1.y : up1.x, u0t = t ? u0.y : u0.x, umt = t ? um.y : um.x;
+      const double flq = t ? fq.y : fq.x, flm = t ? fl.y : fl.x, nu = t ? nuq.y : nuq.x, x = t ? xq.y : xq.x;
+      double v;
+      if (ibs < 0) {
+        const double n = x + (flq - flm) * thq;
+        (t ? nn.y : nn.x) = n;
+        v = c2 * nu - (l1 * umt + (l2 * u0t + l3 * upt));  // the increment first: u's rounding enters once
+        v += cg * n;
+        if (V) {
+          v += (cp * thq) * (t ? pq.y - pm.y : pq.x - pm.x);
+        } else {
+          v += t ? ck * pq.x : -ck * pq.y;
+          if (t == 0) v += mp;
         }
-        if (ibs < 0) { Nu[e].x = nn.x; Nu[e].y = nn.y; }
-        X[e].x = rr.x; X[e].y = rr.y;
-        um = u0; u0 = up1; fl = fq;
-        if (V) pm = pq;
+      } else {
+        const double2 di = a.duib[((size_t)ibs * 3 + fd) * nc + c];
+        v = dt * (t ? di.y : di.x);
       }
+      (t ? rr.y : rr.x) = u0t + v;
+    }
+    if (ibs < 0) { Nu[e].x = nn.x; Nu[e].y = nn.y; }
+    X[e].x = rr.x; X[e].y = rr.y;
+    um = u0; u0 = up1; fl = fq;
+    if (V) pm = pq;
+  }
 }
 // grid: x = (column block, field), y = chunk of levels
 __global__ void __launch_bounds__(128) k_helm_rhs(HelmArgs a, Geo g, const DevScalars *__restrict__ sc) {
@@ -2912,7 +2913,8 @@ __global__ void __launch_bounds__(NTHR, LH_IBDU_MINB) k_ib_du_mx(const double2 *
 // velocities, and the rows go back (B layout for the z pass). Forced points come as
 // records sorted by (plane, row): rec_off[plane * G2 + row] .. rec_off[... + 1];
 // cap [capslot][field][G2][G1] holds the physical u, v, w the x pass captured, in the
-// transform precision (FP32 in the mixed form: the values are FP32 there).
+// transform precision (FP32 in the mixed form: the values are FP32 there). Here the mixed
+// form's kernel; the FP64 form's is k_ib_xforce_fx.
 // ============================================================================
 struct IbRec {
   int i, k;        // 0-based point of the plane: x index, row
@@ -2920,12 +2922,13 @@ struct IbRec {
   long long ref;   // cap offset of u at the reference point (i1, k1, j1)
   double A;
 };
-template <typename T, int N>
-__global__ void __launch_bounds__(NTHR, LH_IBX_MINB) k_ib_xforce(const typename C2<T>::t *__restrict__ A, typename C2<T>::t *__restrict__ B,
-                                                    Geo g, const typename C2<T>::t *__restrict__ twx,
+template <int N>
+__global__ void __launch_bounds__(NTHR, LH_IBX_MINB) k_ib_xforce(const float2 *__restrict__ A, float2 *__restrict__ B,
+                                                    Geo g, const float2 *__restrict__ twx,
                                                     const IbRec *__restrict__ rec, const int *__restrict__ rec_off,
-                                                    const T *__restrict__ cap, const DevScalars *__restrict__ sc) {
-  typedef typename C2<T>::t V;
+                                                    const float *__restrict__ cap, const DevScalars *__restrict__ sc) {
+  typedef float T;
+  typedef float2 V;
   constexpr int PB = 4 * pb_xpass<V>(N);
   constexpr int G1 = N, H = N / 2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -2959,17 +2962,12 @@ __global__ void __launch_bounds__(NTHR, LH_IBX_MINB) k_ib_xforce(const typename 
   V *res = line_fft<true, N, PB, false>(b0, b1, twx);
   V *oth = (res == b0) ? b1 : b0;
   {
-    const double Kibdt = g.Kib / sc->dt;
-    const float Kibdtf = d2f_alu(Kibdt);
+    const float Kibdtf = d2f_alu(g.Kib / sc->dt);
     const int r0 = rec_off[(size_t)pl * G2 + l0], r1 = rec_off[(size_t)pl * G2 + l0 + 2 * npairs];
     for (int e = r0 + threadIdx.x; e < r1; e += blockDim.x) {
       const IbRec R = rec[e];
-      T val;
-      if constexpr (sizeof(T) == 4) {  // FP32 values: one rounding of A u_ref - u (fused), one of the scaling
-        val = Kibdtf * fmaf(d2f_alu(R.A), cap[R.ref], -cap[R.src]);
-      } else {
-        val = Kibdt * (R.A * cap[R.ref] - cap[R.src]);
-      }
+      // one rounding of A u_ref - u (fused), one of the scaling
+      const float val = Kibdtf * fmaf(d2f_alu(R.A), cap[R.ref], -cap[R.src]);
       const int rr = R.k - l0;
       V *z = res + (rr >> 1) * G1 + R.i;
       if (rr & 1) z->y = val;
