@@ -44,7 +44,7 @@ enum {
 };
 
 enum {
-  LH_PREC_FP64 = 0,    /* plain form: every kernel in FP64 */
+  LH_PREC_FP64 = 0,    /* plain form: FP64; transforms in 64-bit block fixed point, no less accurate */
   LH_PREC_MIXED = 1    /* precision form: FP32 transforms/products, FP64 state, solves and (0,0) mode */
 };
 

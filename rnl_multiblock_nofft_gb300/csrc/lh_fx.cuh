@@ -11,7 +11,7 @@
 // multiplies by twiddles stored as w * 2^62 and keeps the high word of the 128-bit product,
 // i.e. divides by 4. s is the largest power of two for which no stage can pass 63 bits
 // (fx_headroom). The quantum of an N-point result is then N * max / 2^63 of the line or
-// finer; the rounding error of a transform, measured over the line shapes of
+// finer (of a line of subnormal values N * 2^-1022 / 2^63); the rounding error of a transform, measured over the line shapes of
 // tests/fx_host_check.cu, is below that of the FP64 Stockham passes at every length.
 // A line that holds an Inf or NaN gives NaN everywhere, as its FP64 transform does.
 #pragma once

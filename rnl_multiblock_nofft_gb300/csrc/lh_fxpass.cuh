@@ -26,11 +26,20 @@ __host__ __device__ constexpr int fx_pbl(int n) { return lh_clamp(fx_pow2(49152 
 __host__ __device__ constexpr size_t fx_smem(int n, int lines) { return (size_t)32 * n * lines; }  // two buffers
 // Threads of a block: as many as the stage with the most butterflies has, so that each stage is
 // one round (a stage of 256 butterflies on 192 threads is two, the second one third full), within
-// the registers of four blocks. ms a step against 192 (384 above a length of 384) everywhere,
-// inverse z / forward z: 384 (256 threads) .822 / 1.072 -> .778 / .939, 192 (256) .400 / .425 ->
-// .380 / .392, 144 (128) .264 / .272 -> .247 / .255, 576 (192, 320) 1.747 / 1.79 -> 1.346 / 1.81.
+// the registers of as many blocks as the SM's shared memory (233472 bytes) holds, four at most.
+// ms a step against 192 threads (384 above a length of 384) everywhere, smooth channels of 385 ... 49
+// levels; only the passes whose threads the rule changes:
+//   length       24     48    144    192    384    576    768   1152
+//   inverse z  .118          .511   .518   .820  2.093  3.371  8.946   192 / 384 threads
+//              .111          .468   .492   .777  1.611  2.699  7.270   the rule
+//   forward z  .074   .169   .506   .548  1.068  2.147
+//              .073   .159   .460   .504   .939  2.161
+//   x                       1.309                5.270
+//                           1.129                5.201
+// The forward z pass of 576 is the one that lost (0.7 %). 256 threads above a length of 384 give 576 forward z
+// 1.883 and x 4.514, but 1152 x 28.99 (25.70) and forward z 11.97 (10.63), and inverse z less everywhere.
 // The x pass keeps 192 up to a length of 384: its instruction issue gains nothing from more warps
-// (384: 192 threads 2.401, 256 2.453; 192: .911, .953), and fewer suit 144 (192 .643, 128 .566).
+// (384: 192 threads 2.401, 256 2.453; 192: .911, .953).
 __host__ __device__ constexpr int fx_threads(int n, int lines, int most = 384) {
   const int f = fx_first(n), s = fx_second(n), l = n / (f * s);
   const int r = l > 1 && l < (f < s ? f : s) ? l : (f < s ? f : s);
@@ -98,7 +107,7 @@ __device__ __forceinline__ void fx_zinv_body(unsigned char *smem, const int4 *__
       [&](int line, int e, fx2 v) { put(e, line, make_double2(fx_out(v.x, sc.S), fx_out(v.y, sc.S))); });
 }
 
-// Inverse z transforms of the velocity planes with the stagger interpolation (k_zinv_nl).
+// Inverse z transforms of the velocity planes with the stagger interpolation (FOU3D.f90:427-474).
 // grid: x = column group, y = level slot, z = field.
 template <int N>
 __global__ void __launch_bounds__(fx_zt(N)) k_zinv_fx(const double2 *__restrict__ u1, const double2 *__restrict__ u2,
@@ -138,7 +147,7 @@ __global__ void __launch_bounds__(fx_zt(N)) k_zinv_fx(const double2 *__restrict_
       });
 }
 
-// plane transform of the leaves and of du's planes (k_spec_zinv)
+// plane transform of the leaves and of du's planes (mixed form: k_spec_zinv2)
 template <int N>
 __global__ void __launch_bounds__(fx_zt(N)) k_spec_zinv_fx(const double2 *__restrict__ spec, double2 *__restrict__ A,
                                                            Geo g, const int4 *__restrict__ tw) {
@@ -245,7 +254,7 @@ __device__ __forceinline__ void fx_zfwd_body(const double2 *__restrict__ B, cons
   }
 }
 
-// Forward z transforms + der_x / der_z (k_zfwd_nl). grid: x = column group, y = level slot; a v
+// Forward z transforms + der_x / der_z (FOU3D.f90:476-593). grid: x = column group, y = level slot; a v
 // level has two products instead of four and takes twice the columns, so that every block
 // carries the same lines.
 template <int N>
@@ -265,7 +274,7 @@ __global__ void __launch_bounds__(fx_ft(N)) k_zfwd_fx(const double2 *__restrict_
   }
 }
 
-// plane transform of the leaves and of du's planes (k_zfwd_spec); B [plane][l][kx]. scale: the
+// plane transform of the leaves and of du's planes (mixed form: k_zfwd_spec2); B [plane][l][kx]. scale: the
 // factor of both transforms (the x passes below leave theirs out)
 template <int N>
 __global__ void __launch_bounds__(fx_zt(N)) k_zfwd_spec_fx(const double2 *__restrict__ B, double2 *__restrict__ spec,
@@ -445,7 +454,7 @@ template <int N, int NL> __host__ __device__ constexpr int fx_xslots() {
 }
 
 // ============================================================================
-// x pass of the substep (k_xpass_nl): inverse transform, products, CFL maxima, forward
+// x pass of the substep: inverse transform, products, CFL maxima, forward
 // transform. The products are formed from the integer fields, normalised by each field's
 // largest value on the line, as the forward transform's first stage reads them.
 // ============================================================================
@@ -591,8 +600,8 @@ __global__ void __launch_bounds__(fx_xt(N)) k_xpass_fx(const double2 *__restrict
 }
 
 // ============================================================================
-// Leaf plane transforms (k_xinv_phys, k_xfwd_phys), the immersed-boundary round trip
-// (k_ib_xforce) and the statistics' plane sums (k_xstats) on the same lines.
+// Leaf plane transforms, the immersed-boundary round trip (mixed form: k_ib_xforce) and the
+// statistics' plane sums (mixed form: k_xstats) on the same lines.
 // ============================================================================
 template <int N>
 __global__ void __launch_bounds__(fx_lt(N)) k_xinv_phys_fx(const double2 *__restrict__ A, double *__restrict__ phys, Geo g,

@@ -1,6 +1,6 @@
 // lh_xpass2.cuh — the x pass of the mixed form as a two-stage transform held in registers.
 //
-// Same work as k_xpass_nl (lh_kernels.cuh) for one level's plane: the inverse x transforms
+// Same work as the FP64 form's k_xpass_fx (lh_fxpass.cuh) for one level's plane: the inverse x transforms
 // (rft, iopt >= 0) of u, v, w row pairs, the physical products of ops_in_planes2
 // (FOU3D.f90:2090-2251), the CFL maxima (dtc_calc) and the forward x transforms (rft,
 // iopt < 0) of the products, with the same A input and B output layouts. Two rows l, l+1 of
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(xp2<N>::NT, xp2<N>::MINB) k_xpass2(const float
 }
 
 // ============================================================================
-// The inverse z pass of the mixed form as a two-stage transform (the work of k_zinv_nl:
+// The inverse z pass of the mixed form as a two-stage transform (the work of k_zinv_fx:
 // stagger interpolation (interp_u/v, FOU3D.f90:427-474) and the inverse z transforms (cft,
 // iopt >= 0) of one field's kx columns at one level, written to A [slot*3 + f][l][kx]).
 // N = ZA * ZB; stage 1: ZB threads per line, each a ZA-point DFT of rows jj + ZB t, gathered
@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(zp2<N>::NT, LH_SPECZ_MINB(N)) k_spec_zinv2(con
 }
 
 // ============================================================================
-// The forward z pass of the mixed form as a two-stage transform (the work of k_zfwd_nl:
+// The forward z pass of the mixed form as a two-stage transform (the work of k_zfwd_fx:
 // forward z transforms (cft, iopt < 0) of the x pass's products and der_x / der_z,
 // FOU3D.f90:476-593, 2253-2272). Per block: KF kx columns of the NP products of one level
 // (u level: uu, uw, vv, ww -> N1xz, N3xz, vvc; v level: uv, wv -> N2xz, uvf, wvf).
@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(zp2<N>::NT, LH_SPECZ_MINB(N)) k_zfwd_spec2(con
 
 // ============================================================================
 // The x pass of the mixed form at the long lengths (576, 768, 1152) as a three-stage register
-// transform, N = XA * XM * 8, one row pair per block (the work of k_xpass_nl, same A and B
+// transform, N = XA * XM * 8, one row pair per block (the work of k_xpass_fx, same A and B
 // layouts). Stages, each a register DFT between padded shared-memory lines:
 //   inverse: XA-point DFTs gathered straight from A (Hermitian completion) -> XM-point DFTs ->
 //            8-point DFTs fused with the products, the CFL maxima and the forward 8-point DFTs
