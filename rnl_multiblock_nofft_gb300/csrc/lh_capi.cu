@@ -40,7 +40,7 @@ struct lh_handle {
   void *ysf, *ysv;  // FP32 scratch of the mixed-form solves (u and w; v)
   void *N1xz, *N2xz, *N3xz, *uvf, *vvc, *wvf;  // transform outputs, transform precision
   double *a3s, *a3v, *mfw;
-  double2 *faces;  // k_press_rhs / k_press_corr: v's face below each chunk of levels
+  double2 *faces;  // k_press_rhs / k_press_corr: v's face below each chunk of levels (behind psi)
   void *A, *B, *twx, *twz, *twx64, *twz64;
   size_t Abytes, Bbytes;
   long long graph_nodes_per_step;
@@ -426,10 +426,12 @@ extern "C" int lh_create(const lh_config *cfg, lh_handle **out) {
   // a3s: the FP64 solves' upper factors; in the mixed form the previous nonlinear term of mode
   // (0,0) in FP64 (k_helm00_pcr: 6 x nu doubles; nc >= 8 always)
   const size_t split = h->prec == LH_PREC_FP64 && g.nvc < LH_HELM_SPLIT ? 2 : 1;  // k_helm_sweep64: factors per field and part
-  ZA(h->psi, cz * g.np * nc); ZA(h->a3s, split * split * sizeof(double) * nu * nc); ZA(h->a3v, split * sizeof(double) * nv * nc);
+  // psi, and behind it the faces of the split pressure step (the segments of a multiblock channel can be
+  // more than the transforms' scratch holds)
+  ZA(h->psi, cz * g.np * nc + (g.nvc < LH_PRESS_SPLIT_COLS ? press_faces_bytes(g) : 0));
+  h->faces = h->psi + g.np * nc;
+  ZA(h->a3s, split * split * sizeof(double) * nu * nc); ZA(h->a3v, split * sizeof(double) * nv * nc);
   ZA(h->mfw, sizeof(double) * 6 * (size_t)(g.nn + 3));
-  // (an array of its own: the segments of a multiblock channel can be more than A holds)
-  if (g.nvc < LH_PRESS_SPLIT_COLS) ZA(h->faces, press_faces_bytes(g));
   h->Abytes = h->Bbytes = 0;
   for (int vi = 0; vi < h->nviews; ++vi) {
     const size_t nuv = vsl[vi][0].size(), nvv = vsl[vi][1].size();
@@ -707,7 +709,7 @@ extern "C" int lh_destroy(lh_handle *h) {
   if (!h) return LH_EINVAL;
   if (h->graph_ready) { cudaGraphExecDestroy(h->gexec); cudaGraphDestroy(h->graph); }
   void *bufs[] = {h->u1, h->u2, h->u3, h->p, h->Nu1, h->Nu2, h->Nu3, h->dg1, h->dg2, h->dg3, h->ysf, h->N1xz, h->N2xz, h->N3xz, h->uvf, h->vvc,
-                  h->wvf, h->psi, h->a3s, h->mfw, h->faces, h->A, h->B, h->twx, h->twz, h->twx64, h->twz64, h->geo_pool, h->geo_poolf, h->sc, h->stage,
+                  h->wvf, h->psi, h->a3s, h->mfw, h->A, h->B, h->twx, h->twz, h->twx64, h->twz64, h->geo_pool, h->geo_poolf, h->sc, h->stage,
                   h->d_ibslot_u, h->d_ibslot_v, h->d_iblev, h->d_lev2cap_u,
                   h->d_lev2cap_v, h->d_ibrec, h->d_iboff, h->cap, h->duib, h->d_terms, h->d_wb, h->d_lid, h->d_tmap,
                   h->d_slotq, h->d_capv, h->d_vcol, h->d_bcols, h->twv[1][0], h->twv[1][1],
